@@ -1,0 +1,65 @@
+// Builders of the LOD brick cache (r3d_build.cu) and the byte-row loads that
+// device-side builders share.
+#pragma once
+
+#include "r3d_march.cuh"
+
+namespace r3d {
+
+// Bytes [x, x + 4) of a row of n bytes, zero past its end.  VEC: the row and
+// x are 4-byte aligned and n a multiple of 4; else two aligned words are
+// shifted together, and only words that hold a byte of the row are read.
+template <bool VEC>
+__device__ __forceinline__ uint32_t load4(const uint8_t *__restrict__ row, uint32_t x, uint32_t n) {
+  if (x >= n) return 0u;
+  if (VEC) return __ldg(reinterpret_cast<const uint32_t *>(row + x));
+  const uintptr_t a = (uintptr_t)(row + x), last = (uintptr_t)(row + n - 1u);
+  const uint32_t *w = reinterpret_cast<const uint32_t *>(a & ~(uintptr_t)3);
+  const uint32_t lo = __ldg(w);
+  const uint32_t hi = (uintptr_t)(w + 1) <= last ? __ldg(w + 1) : 0u;
+  const uint32_t v = __funnelshift_r(lo, hi, 8u * (uint32_t)(a & 3u));
+  const uint32_t left = n - x;
+  return left >= 4u ? v : v & (0xFFFFFFFFu >> (8u * (4u - left)));
+}
+
+// Bytes [x, x + 8) likewise (VEC: 8-byte aligned, n a multiple of 8).
+template <bool VEC>
+__device__ __forceinline__ uint2 load8(const uint8_t *__restrict__ row, uint32_t x, uint32_t n) {
+  if (VEC)
+    return x < n ? __ldg(reinterpret_cast<const uint2 *>(row + x)) : make_uint2(0u, 0u);
+  return make_uint2(load4<false>(row, x, n), load4<false>(row, x + 4u, n));
+}
+
+// the largest of the four bytes of w
+__device__ __forceinline__ uint32_t max_byte(uint32_t w) {
+  w = __vmaxu4(w, w >> 16);
+  return max(w & 0xFFu, (w >> 8) & 0xFFu);
+}
+
+// One pyramid level as a source of bricks: its bytes and extent, its brick
+// grid, and the first job of the level in the job list.
+struct LevelSrc {
+  const uint8_t *p;
+  uint32_t ex, ey, ez;
+  uint32_t bdx, bdy;
+  uint32_t job0;
+};
+
+// 2x box reduction of a level (sx, sy, sz) to dst (dx, dy, dz: multiples of
+// 128, dst null: none) and, with vmax (zeroed by the caller), the maximum of
+// every 128^3 brick of the source (bdx * bdy * ... entries).
+cudaError_t launch_level_down(const uint8_t *src, uint32_t sx, uint32_t sy, uint32_t sz,
+                              uint8_t *dst, uint32_t dx, uint32_t dy, uint32_t dz, uint32_t *vmax,
+                              uint32_t bdx, uint32_t bdy, cudaStream_t st);
+// Slots from bricks of pyramid levels: job j puts brick brick[j] of the level
+// whose job range holds j into slot slot[j] (null: j): its bytes (pool), quad
+// words and block maxima, each left out when null.
+cudaError_t launch_slot_fill(const LevelSrc *lev, uint32_t nlev, const uint32_t *brick,
+                             const uint32_t *slot, uint32_t njobs, uint8_t *pool, uint32_t *quad,
+                             uint8_t *bmax, cudaStream_t st);
+// Quad words and block maxima of slots slot[0..njobs) (null: 0..njobs) of a
+// pool; the source slots may be another pool than the tables' (same index).
+cudaError_t launch_slot_tables(const uint8_t *pool, const uint32_t *slot, uint32_t njobs,
+                               uint32_t *quad, uint8_t *bmax, cudaStream_t st);
+
+}  // namespace r3d

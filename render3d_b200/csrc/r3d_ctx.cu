@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "r3d_build.cuh"
 #include "r3d_internal.h"
 
 namespace r3d {
@@ -35,6 +36,15 @@ bool is_device_ptr(const void *p) {
   return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
+bool readable_in_place(const r3d_cuda_ctx *c, const void *p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeDevice && a.device == c->device;
+}
+
 // ------------------------------------------------------------- builders
 
 // 2x box reduction with clamped source coordinates: (sum + 4) / 8
@@ -51,24 +61,6 @@ __global__ void k_downsample_clamp(const uint8_t *__restrict__ src, uint32_t sx,
       uint32_t xx = min(2u * x + (k & 1u), sx - 1u), yy = min(2u * y + ((k >> 1) & 1u), sy - 1u),
                zz = min(2u * z + (k >> 2), sz - 1u);
       sum += src[((size_t)zz * sy + yy) * sx + xx];
-    }
-    dst[i] = (uint8_t)(sum >> 3);
-  }
-}
-
-// 2x box reduction reading zeros outside the source extent (brick pyramid)
-__global__ void k_downsample_zero(const uint8_t *__restrict__ src, uint32_t sx, uint32_t sy,
-                                  uint32_t sz, uint8_t *__restrict__ dst, uint32_t dx,
-                                  uint32_t dy, uint32_t dz) {
-  size_t n = (size_t)dx * dy * dz;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    uint32_t x = (uint32_t)(i % dx), y = (uint32_t)((i / dx) % dy), z = (uint32_t)(i / dx / dy);
-    uint32_t sum = 4u;
-#pragma unroll
-    for (uint32_t k = 0; k < 8u; k++) {
-      uint32_t xx = 2u * x + (k & 1u), yy = 2u * y + ((k >> 1) & 1u), zz = 2u * z + (k >> 2);
-      if (xx < sx && yy < sy && zz < sz) sum += src[((size_t)zz * sy + yy) * sx + xx];
     }
     dst[i] = (uint8_t)(sum >> 3);
   }
@@ -108,82 +100,6 @@ __global__ void k_occ_dilate(const uint8_t *__restrict__ raw, uint8_t *__restric
           m = max(m, (uint32_t)raw[((size_t)zz * oy + yy) * ox + xx]);
         }
     dil[i] = (uint8_t)m;
-  }
-}
-
-// Maximum of each 128^3 brick of a level (zero outside the level's extent).
-// One block per brick.
-__global__ void k_brick_max(const uint8_t *__restrict__ lev, uint32_t ex, uint32_t ey,
-                            uint32_t ez, uint32_t bdx, uint32_t bdy, uint32_t *__restrict__ out) {
-  uint32_t bi = blockIdx.x;
-  uint32_t bx = bi % bdx, by = (bi / bdx) % bdy, bz = bi / bdx / bdy;
-  uint32_t m = 0;
-  for (uint32_t r = threadIdx.x; r < 128u * 128u; r += blockDim.x) {
-    uint32_t y = by * 128u + (r & 127u), z = bz * 128u + (r >> 7);
-    if (y >= ey || z >= ez) continue;
-    const uint8_t *row = lev + ((size_t)z * ey + y) * ex;
-    uint32_t x0 = bx * 128u, x1 = min(x0 + 128u, ex);
-    for (uint32_t x = x0; x < x1; x++) m = max(m, (uint32_t)row[x]);
-  }
-  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-  __shared__ uint32_t wm[32];
-  if ((threadIdx.x & 31u) == 0) wm[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t r = 0;
-    for (uint32_t w = 0; w < blockDim.x / 32u; w++) r = max(r, wm[w]);
-    out[bi] = r;
-  }
-}
-
-// Copies bricks into their slots: job j copies brick src_brick[j] (linear
-// index in the level's brick grid) into slot dst_slot[j]; zero outside the
-// level's extent.  Grid: (128 z-slices, jobs).
-__global__ void k_brick_copy(const uint8_t *__restrict__ lev, uint32_t ex, uint32_t ey,
-                             uint32_t ez, uint32_t bdx, uint32_t bdy,
-                             const uint32_t *__restrict__ src_brick,
-                             const uint32_t *__restrict__ dst_slot, uint8_t *__restrict__ pool) {
-  uint32_t j = blockIdx.y, zl = blockIdx.x;
-  uint32_t bi = src_brick[j];
-  uint32_t bx = bi % bdx, by = (bi / bdx) % bdy, bz = bi / bdx / bdy;
-  uint8_t *dst = pool + (size_t)dst_slot[j] * (128u * 128u * 128u) + (size_t)zl * 16384u;
-  uint32_t z = bz * 128u + zl;
-  for (uint32_t r = threadIdx.x; r < 128u * 128u; r += blockDim.x) {
-    uint32_t yl = r >> 7, xl = r & 127u;
-    uint32_t y = by * 128u + yl, x = bx * 128u + xl;
-    uint8_t v = 0;
-    if (x < ex && y < ey && z < ez) v = lev[((size_t)z * ey + y) * ex + x];
-    dst[r] = v;
-  }
-}
-
-// Per-slot table of dilated 8^3 block maxima: entry (bz, by, bx) of slot s
-// is the max over voxels [8b, min(8b+8, 127)] on each axis.  One block per
-// slot, one thread per table entry.
-__global__ void k_slot_blockmax(const uint8_t *__restrict__ pool, uint8_t *__restrict__ out) {
-  const uint8_t *g = pool + (size_t)blockIdx.x * (128u * 128u * 128u);
-  for (uint32_t e = threadIdx.x; e < 4096u; e += blockDim.x) {
-    uint32_t bx = e & 15u, by = (e >> 4) & 15u, bz = e >> 8;
-    uint32_t m = 0;
-    for (uint32_t z = bz * 8u; z <= min(bz * 8u + 8u, 127u); z++)
-      for (uint32_t y = by * 8u; y <= min(by * 8u + 8u, 127u); y++) {
-        const uint8_t *row = g + ((size_t)z << 14) + ((size_t)y << 7);
-        for (uint32_t x = bx * 8u; x <= min(bx * 8u + 8u, 127u); x++)
-          m = max(m, (uint32_t)row[x]);
-      }
-    out[(size_t)blockIdx.x * 4096u + e] = (uint8_t)m;
-  }
-}
-
-// Quad words of every slot (DevBricks::quad); one thread per texel.
-__global__ void k_slot_quads(const uint8_t *__restrict__ pool, uint32_t *__restrict__ quad,
-                             size_t n) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const uint32_t x = (uint32_t)(i & 127u), y = (uint32_t)((i >> 7) & 127u);
-    const size_t dx = x < 127u ? 1u : 0u, dy = y < 127u ? 128u : 0u;
-    quad[i] = (uint32_t)pool[i] | ((uint32_t)pool[i + dx] << 8) | ((uint32_t)pool[i + dy] << 16) |
-              ((uint32_t)pool[i + dy + dx] << 24);
   }
 }
 
@@ -454,33 +370,60 @@ static int decode_header(r3d_cuda_ctx *c, const uint32_t *page, uint32_t words, 
   return R3D_OK;
 }
 
-// (Re)builds the block-maximum table of the context's slot pool.
-int build_blockmax(r3d_cuda_ctx *c) {
-  if (c->defer_tables) return R3D_OK;
-  cudaFree(c->bmax);
-  c->bmax = nullptr;
-  size_t n = (size_t)(c->nslots ? c->nslots : 1u) * 4096u;
-  R3D_CUDA_TRY(c, cudaMalloc(&c->bmax, n));
-  R3D_CUDA_TRY(c, cudaMemsetAsync(c->bmax, 0, n, c->stream));
-  cudaFree(c->quad);
-  c->quad = nullptr;
-  for (int i = 0; i < 4; i++) {  // overlays follow the old slot assignment
+// Device buffers of a brick cache outlive a rebuild of about the same size:
+// one of at least `need` and less than twice that many bytes is used again
+// (a 1024^3 cache's cudaMalloc and cudaFree calls took 10 ms of a rebuild's
+// 23), any other is replaced.  Frames in flight on other streams may still
+// read a kept buffer, so the device is idle before it is written again, as
+// cudaFree leaves it too.
+static bool keeps(const void *p, size_t cap, size_t need) { return p && cap >= need && need > cap / 2; }
+
+template <class T>
+static cudaError_t reserve(T *&p, size_t &cap, size_t need) {
+  if (keeps(p, cap, need)) return cudaDeviceSynchronize();
+  cudaFree(p);
+  p = nullptr;
+  cap = 0;
+  const cudaError_t e = cudaMalloc(&p, need);
+  if (e == cudaSuccess) cap = need;
+  return e;
+}
+
+// Room for the per-slot tables (block maxima, quad words) of c->nslots
+// slots; overlays follow the old slot assignment and go.
+static int reserve_tables(r3d_cuda_ctx *c) {
+  for (int i = 0; i < 4; i++) {
     cudaFree(c->ovl_quad[i]);
     c->ovl_quad[i] = nullptr;
     c->br.ovl[i] = nullptr;
     c->ovl_src_on[i] = false;  // a new cache detaches CPU-sourced atlases
     c->ovl_key[i].clear();
   }
-  const size_t nq = (size_t)(c->nslots ? c->nslots : 1u) * (128u * 128u * 128u);
-  R3D_CUDA_TRY(c, cudaMalloc(&c->quad, nq * sizeof(uint32_t)));
-  if (c->nslots) {
-    k_slot_blockmax<<<c->nslots, 256, 0, c->stream>>>(c->pool, c->bmax);
-    k_slot_quads<<<grid_for(nq), 256, 0, c->stream>>>(c->pool, c->quad, nq);
-    R3D_CUDA_TRY(c, cudaGetLastError());
-  }
+  c->br.bmax = nullptr;
+  c->br.quad = nullptr;
+  const size_t n = c->nslots ? c->nslots : 1u;
+  R3D_CUDA_TRY(c, reserve(c->bmax, c->bmax_cap, n * 4096u));
+  R3D_CUDA_TRY(c, reserve(c->quad, c->quad_cap, n * (128u * 128u * 128u) * sizeof(uint32_t)));
+  if (!c->nslots) R3D_CUDA_TRY(c, cudaMemsetAsync(c->bmax, 0, 4096u, c->stream));
+  return R3D_OK;
+}
+
+// (Re)builds the per-slot tables of the context's slot pool.
+int build_blockmax(r3d_cuda_ctx *c) {
+  if (c->defer_tables) return R3D_OK;
+  const int rc = reserve_tables(c);
+  if (rc != R3D_OK) return rc;
+  R3D_CUDA_TRY(c, launch_slot_tables(c->pool, nullptr, c->nslots, c->quad, c->bmax, c->stream));
   R3D_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   c->br.bmax = c->bmax;
   c->br.quad = c->quad;
+  return R3D_OK;
+}
+
+int replace_pool(r3d_cuda_ctx *c, uint32_t nslots) {
+  c->br.pool = nullptr;
+  R3D_CUDA_TRY(c, reserve(c->pool, c->pool_cap, (size_t)(nslots ? nslots : 1u) * (128u * 128u * 128u)));
+  c->br.pool = c->pool;
   return R3D_OK;
 }
 
@@ -520,36 +463,49 @@ int r3d_cuda_bricks_build(r3d_cuda_ctx *c, const r3d_volume_desc *d, const uint8
     lev_total += ((size_t)E[l][0] * E[l][1] * E[l][2] + 255) & ~(size_t)255;
     nb_total += bd[l][0] * bd[l][1] * bd[l][2];
   }
+  // the level buffer holds levels 1.. and, when the voxels are not on this
+  // device, level 0; a device volume is read where it is
+  const bool dev_in = readable_in_place(c, voxels);
+  if (dev_in) {
+    const size_t skip = nlev > 1u ? lev_off[1] : lev_total;
+    for (uint32_t l = 1; l < nlev; l++) lev_off[l] -= skip;
+    lev_total -= skip;
+  }
   uint32_t words = R3D_BRICK_PAGE_HEADER + nb_total;
   uint8_t *lev = nullptr;
   uint32_t *dmax = nullptr, *jobs = nullptr;
   uint8_t *pool = nullptr;
   uint32_t *page = nullptr;
+  size_t pool_bytes = 0;
   std::vector<uint32_t> hmax(nb_total), hpage(words, R3D_BRICK_ABSENT);
-  std::vector<uint32_t> src_brick, dst_slot;
+  std::vector<uint32_t> src_brick;
+  LevelSrc src[16];
   int rc = R3D_OK;
-  cudaError_t e = cudaMalloc(&lev, lev_total);
-  if (e == cudaSuccess) e = cudaMalloc(&dmax, (size_t)nb_total * 4);
+  // level buffer, brick maxima, brick list: one allocation
+  const size_t max_off = (lev_total + 255) & ~(size_t)255, job_off = max_off + (size_t)nb_total * 4;
+  cudaError_t e = cudaMalloc(&lev, job_off + (size_t)nb_total * 4);
   if (e != cudaSuccess) {
     rc = cuda_fail(c, e, "bricks_build: cudaMalloc levels");
     goto out;
   }
-  e = cudaMemcpyAsync(lev, voxels, (size_t)nx * ny * nz, cudaMemcpyDefault, st);
-  for (uint32_t l = 1; l < nlev && e == cudaSuccess; l++) {
-    size_t n = (size_t)E[l][0] * E[l][1] * E[l][2];
-    k_downsample_zero<<<grid_for(n), 256, 0, st>>>(lev + lev_off[l - 1], E[l - 1][0], E[l - 1][1],
-                                                   E[l - 1][2], lev + lev_off[l], E[l][0], E[l][1],
-                                                   E[l][2]);
-    e = cudaGetLastError();
-  }
+  dmax = (uint32_t *)(lev + max_off);
+  jobs = (uint32_t *)(lev + job_off);
+  e = cudaMemsetAsync(dmax, 0, (size_t)nb_total * 4, st);
+  if (e == cudaSuccess && !dev_in)
+    e = cudaMemcpyAsync(lev, voxels, (size_t)nx * ny * nz, cudaMemcpyDefault, st);
   {
+    // each level is read once: the next one and the level's brick maxima
     uint32_t moff = 0;
-    for (uint32_t l = 0; l < nlev && e == cudaSuccess; l++) {
-      uint32_t nb = bd[l][0] * bd[l][1] * bd[l][2];
-      k_brick_max<<<nb, 256, 0, st>>>(lev + lev_off[l], E[l][0], E[l][1], E[l][2], bd[l][0],
-                                      bd[l][1], dmax + moff);
-      e = cudaGetLastError();
-      moff += nb;
+    for (uint32_t l = 0; l < nlev; l++) {
+      src[l] = {l == 0 && dev_in ? voxels : lev + lev_off[l], E[l][0], E[l][1], E[l][2],
+                bd[l][0], bd[l][1], 0u};
+      uint32_t o[3];
+      for (int a = 0; a < 3; a++) o[a] = l + 1u < nlev ? E[l + 1][a] : (bd[l][a] + 1u) / 2u * 128u;
+      if (e == cudaSuccess)
+        e = launch_level_down(src[l].p, E[l][0], E[l][1], E[l][2],
+                              l + 1u < nlev ? lev + lev_off[l + 1] : nullptr, o[0], o[1], o[2],
+                              dmax + moff, bd[l][0], bd[l][1], st);
+      moff += bd[l][0] * bd[l][1] * bd[l][2];
     }
   }
   if (e == cudaSuccess)
@@ -572,10 +528,12 @@ int r3d_cuda_bricks_build(r3d_cuda_ctx *c, const r3d_volume_desc *d, const uint8
       hpage[4 + 4 * l] = R3D_BRICK_PAGE_HEADER + off;
       hpage[5 + 4 * l] = bd[l][0] | (bd[l][1] << 10) | (bd[l][2] << 20);
       hpage[6 + 4 * l] = 1u << l;
+      src[l].job0 = slot;
       for (uint32_t bi = 0; bi < nb; bi++) {
         uint32_t m = hmax[off + bi];
         if (m >= min_max) {
           hpage[R3D_BRICK_PAGE_HEADER + off + bi] = slot | (m << 24);
+          src_brick.push_back(bi);
           slot++;
         }
       }
@@ -586,67 +544,32 @@ int r3d_cuda_bricks_build(r3d_cuda_ctx *c, const r3d_volume_desc *d, const uint8
       goto out;
     }
     uint32_t nslots = slot;
-    size_t pool_bytes = (size_t)(nslots ? nslots : 1u) * (128u * 128u * 128u);
-    e = cudaMalloc(&pool, pool_bytes);
+    DevBricks b;
+    rc = decode_header(c, hpage.data(), words, nslots, b);
+    if (rc != R3D_OK) goto out;
+    // the pool and the page table: kept when about this size, else allocated
+    // before the old ones go
+    pool_bytes = (size_t)(nslots ? nslots : 1u) * (128u * 128u * 128u);
+    if (!keeps(c->pool, c->pool_cap, pool_bytes)) e = cudaMalloc(&pool, pool_bytes);
     if (e == cudaSuccess) e = cudaMalloc(&page, (size_t)words * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&jobs, (size_t)(nslots ? nslots : 1u) * 8);
     if (e != cudaSuccess) {
       rc = cuda_fail(c, e, "bricks_build: cudaMalloc pool");
       goto out;
     }
-    off = 0;
-    uint32_t joff = 0;
-    std::vector<uint32_t> hj;
-    hj.reserve((size_t)nslots * 2);
-    std::vector<uint32_t> lvl_count(nlev, 0);
-    for (uint32_t l = 0; l < nlev; l++) {
-      uint32_t nb = bd[l][0] * bd[l][1] * bd[l][2];
-      for (uint32_t bi = 0; bi < nb; bi++) {
-        uint32_t en = hpage[R3D_BRICK_PAGE_HEADER + off + bi];
-        if (en != R3D_BRICK_ABSENT) {
-          src_brick.push_back(bi);
-          dst_slot.push_back(en & 0xFFFFFFu);
-          lvl_count[l]++;
-        }
-      }
-      off += nb;
+    c->have_bricks = false;
+    if (pool) {
+      cudaFree(c->pool);
+      c->pool = pool;
+      c->pool_cap = pool_bytes;
+      pool = nullptr;
+    } else {
+      e = cudaDeviceSynchronize();  // frames on other streams may read the old slots
     }
-    if (nslots) {
-      e = cudaMemcpyAsync(jobs, src_brick.data(), (size_t)nslots * 4, cudaMemcpyHostToDevice, st);
-      if (e == cudaSuccess)
-        e = cudaMemcpyAsync(jobs + nslots, dst_slot.data(), (size_t)nslots * 4,
-                            cudaMemcpyHostToDevice, st);
-    }
-    for (uint32_t l = 0; l < nlev && e == cudaSuccess; l++) {
-      uint32_t n = lvl_count[l];
-      if (!n) continue;
-      for (uint32_t j0 = 0; j0 < n && e == cudaSuccess; j0 += 65535u) {
-        uint32_t nj = min(n - j0, 65535u);
-        k_brick_copy<<<dim3(128, nj), 256, 0, st>>>(lev + lev_off[l], E[l][0], E[l][1], E[l][2],
-                                                    bd[l][0], bd[l][1], jobs + joff + j0,
-                                                    jobs + nslots + joff + j0, pool);
-        e = cudaGetLastError();
-      }
-      joff += n;
-    }
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(page, hpage.data(), (size_t)words * 4, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) {
-      rc = cuda_fail(c, e, "bricks_build: slot copy");
-      goto out;
-    }
-    DevBricks b;
-    rc = decode_header(c, hpage.data(), words, nslots, b);
-    if (rc != R3D_OK) goto out;
-    b.page = page;
-    b.pool = pool;
     cudaFree(c->page);
-    cudaFree(c->pool);
     c->page = page;
-    c->pool = pool;
     page = nullptr;
-    pool = nullptr;
+    b.page = c->page;
+    b.pool = c->pool;
     c->page_words = words;
     c->nslots = nslots;
     c->abpa = atlas_bpa(nslots);
@@ -654,24 +577,43 @@ int r3d_cuda_bricks_build(r3d_cuda_ctx *c, const r3d_volume_desc *d, const uint8
     c->shape[1] = ny;
     c->shape[2] = nz;
     c->br = b;
-    c->have_bricks = false;
-    // the display filter, before the tables that derive from the slots (a
-    // build whose pool becomes a streaming store stays unfiltered: its
-    // bricks are filtered when uploaded)
-    if (!c->defer_tables && postfilter_on(c, 0u)) {
+    // the display filter comes before the tables that derive from the slots
+    // (a build whose pool becomes a streaming store stays unfiltered: its
+    // bricks are filtered when uploaded); without it one pass over the
+    // levels fills the slots and their tables
+    const bool filter = !c->defer_tables && postfilter_on(c, 0u), fused = !c->defer_tables && !filter;
+    if (fused) {
+      rc = reserve_tables(c);
+      if (rc != R3D_OK) goto out;
+    }
+    if (e == cudaSuccess && nslots)
+      e = cudaMemcpyAsync(jobs, src_brick.data(), (size_t)nslots * 4, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess && nslots)
+      e = launch_slot_fill(src, nlev, jobs, nullptr, nslots, c->pool, fused ? c->quad : nullptr,
+                           fused ? c->bmax : nullptr, st);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(c->page, hpage.data(), (size_t)words * 4, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) {
+      rc = cuda_fail(c, e, "bricks_build: slots");
+      goto out;
+    }
+    if (fused) {
+      c->br.bmax = c->bmax;
+      c->br.quad = c->quad;
+    }
+    if (filter) {
       std::vector<uint32_t> all(nslots);
       for (uint32_t s = 0; s < nslots; s++) all[s] = s;
       rc = postfilter_slots(c, 0u, c->pool, all.data(), nslots);
       if (rc != R3D_OK) goto out;
     }
-    rc = build_blockmax(c);
+    if (!fused) rc = build_blockmax(c);
     if (rc != R3D_OK) goto out;
     c->have_bricks = true;
   }
 out:
   cudaFree(lev);
-  cudaFree(dmax);
-  cudaFree(jobs);
   cudaFree(pool);
   cudaFree(page);
   return rc;
@@ -706,6 +648,7 @@ int r3d_cuda_bricks_load(r3d_cuda_ctx *c, const uint32_t *page, uint32_t page_wo
   cudaFree(c->pool);
   c->page = dpage;
   c->pool = dpool;
+  c->pool_cap = pool_bytes;
   c->page_words = page_words;
   c->nslots = nslots;
   c->abpa = atlas_bpa(nslots);

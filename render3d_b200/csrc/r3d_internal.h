@@ -26,6 +26,7 @@ struct r3d_cuda_ctx {
   uint8_t *pool = nullptr;
   uint8_t *bmax = nullptr;  // per-slot dilated 8^3 block maxima (4096 B/slot)
   uint32_t *quad = nullptr;  // per-slot quad words (DevBricks::quad)
+  size_t pool_cap = 0, bmax_cap = 0, quad_cap = 0;  // bytes of the three
   uint32_t *ovl_quad[4] = {nullptr, nullptr, nullptr, nullptr};  // overlay atlases
   // CPU-sourced atlases: the attached source, each slot's content key and
   // the staging slots (pinned host and device) of one sync round
@@ -184,6 +185,8 @@ namespace r3d {
 int fail(r3d_cuda_ctx *c, int code, const char *fmt, ...);
 int cuda_fail(r3d_cuda_ctx *c, cudaError_t e, const char *what);
 bool is_device_ptr(const void *p);
+// memory of the context's own device, which its kernels can read directly
+bool readable_in_place(const r3d_cuda_ctx *c, const void *p);
 
 // A copy in either direction (host or device source) ordered on stream s and
 // complete on return.  Uploads go through here rather than cudaMemcpy on the
@@ -238,6 +241,8 @@ cudaError_t launch_view(const r3d_cuda_ctx *c, const r3d_frame_params &pc, uint8
 // context's slot pool (dropping its overlays); atlas bricks per axis of a
 // pool of nslots slots.
 int build_blockmax(r3d_cuda_ctx *c);
+// A slot pool of nslots slots in place of the context's (contents undefined).
+int replace_pool(r3d_cuda_ctx *c, uint32_t nslots);
 // Drops the streaming state (host store, shadows, LRU).
 void stream_reset(r3d_cuda_ctx *c);
 // The display filter: whether it changes target t (0 CT, 1 ink atlas, 2 3D

@@ -12,20 +12,10 @@
 
 #include <vector>
 
+#include "r3d_build.cuh"
 #include "r3d_internal.h"
 
 namespace r3d {
-
-// Defined in r3d_ctx.cu.
-__global__ void k_downsample_zero(const uint8_t *__restrict__ src, uint32_t sx, uint32_t sy,
-                                  uint32_t sz, uint8_t *__restrict__ dst, uint32_t dx,
-                                  uint32_t dy, uint32_t dz);
-__global__ void k_brick_copy(const uint8_t *__restrict__ lev, uint32_t ex, uint32_t ey,
-                             uint32_t ez, uint32_t bdx, uint32_t bdy,
-                             const uint32_t *__restrict__ src_brick,
-                             const uint32_t *__restrict__ dst_slot, uint8_t *__restrict__ pool);
-__global__ void k_slot_quads(const uint8_t *__restrict__ pool, uint32_t *__restrict__ quad,
-                             size_t n);
 
 // Level l of a label volume: the level-0 voxel at (x, y, z) << l, zero
 // outside the volume (coarse label bricks stride-sample the paint grid,
@@ -54,13 +44,9 @@ static unsigned ovl_grid(size_t n) {
   return (unsigned)(b < 148u * 64u ? (b ? b : 1) : 148u * 64u);
 }
 
-// Converts a byte pool (device) into overlay atlas `which`.
-static int overlay_quads(r3d_cuda_ctx *c, uint32_t which, const uint8_t *pool) {
-  const size_t n = (size_t)(c->nslots ? c->nslots : 1u) * (128u * 128u * 128u);
-  uint32_t *q = nullptr;
-  R3D_CUDA_TRY(c, cudaMalloc(&q, n * sizeof(uint32_t)));
-  if (c->nslots) k_slot_quads<<<ovl_grid(n), 256, 0, c->stream>>>(pool, q, n);
-  cudaError_t e = cudaGetLastError();
+// The quad words q (being written on the context's stream, launch status e)
+// become overlay atlas `which`.
+static int adopt_overlay(r3d_cuda_ctx *c, uint32_t which, uint32_t *q, cudaError_t e) {
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) {
     cudaFree(q);
@@ -71,6 +57,15 @@ static int overlay_quads(r3d_cuda_ctx *c, uint32_t which, const uint8_t *pool) {
   c->br.ovl[which] = q;
   if (c->ovl_src_on[which]) c->ovl_key[which].assign(c->nslots, UINT64_MAX);  // replaced content
   return R3D_OK;
+}
+
+// Converts a byte pool (device) into overlay atlas `which`.
+static int overlay_quads(r3d_cuda_ctx *c, uint32_t which, const uint8_t *pool) {
+  const size_t n = (size_t)(c->nslots ? c->nslots : 1u) * (128u * 128u * 128u);
+  uint32_t *q = nullptr;
+  R3D_CUDA_TRY(c, cudaMalloc(&q, n * sizeof(uint32_t)));
+  const cudaError_t e = launch_slot_tables(pool, nullptr, c->nslots, q, nullptr, c->stream);
+  return adopt_overlay(c, which, q, e);
 }
 
 // overlay_quads through the display filter when it targets the atlas (ink:
@@ -206,10 +201,9 @@ int r3d_cuda_bricks_atlas_sync(r3d_cuda_ctx *c, uint32_t which, uint32_t budget,
   R3D_CUDA_TRY(c, cudaMemcpyAsync(c->ovl_stage_dev, c->ovl_stage, (size_t)n * kSlotTexels,
                                   cudaMemcpyHostToDevice, c->stream));
   for (uint32_t i = 0; i < n; i++)  // that slot's overlay words
-    k_slot_quads<<<ovl_grid(kSlotTexels), 256, 0, c->stream>>>(
-        c->ovl_stage_dev + (size_t)i * kSlotTexels, c->ovl_quad[which] + (size_t)sel[i] * kSlotTexels,
-        kSlotTexels);
-  R3D_CUDA_TRY(c, cudaGetLastError());
+    R3D_CUDA_TRY(c, launch_slot_tables(c->ovl_stage_dev + (size_t)i * kSlotTexels, nullptr, 1u,
+                                       c->ovl_quad[which] + (size_t)sel[i] * kSlotTexels, nullptr,
+                                       c->stream));
   for (uint32_t i = 0; i < n; i++) c->ovl_key[which][sel[i]] = key[i];
   if (synced) *synced = n;
   return R3D_OK;
@@ -244,71 +238,82 @@ int r3d_cuda_bricks_overlay_build(r3d_cuda_ctx *c, uint32_t which, const r3d_vol
   R3D_CUDA_TRY(c, cudaStreamSynchronize(st));
   const DevBricks &br = c->br;
   const uint32_t nlev = br.nlev, nx = d->nx, ny = d->ny, nz = d->nz;
-  // level extents as the CT pyramid's: level 0 the volume, level l >= 1 the
-  // zero-padded brick grid
-  uint32_t E[16][3];
+  // level extents as the CT pyramid's: level 0 the volume (read where it is
+  // when it lies on this device), level l >= 1 the zero-padded brick grid
+  const bool dev_in = readable_in_place(c, voxels);
+  LevelSrc src[16];
   size_t lev_off[16] = {0}, lev_total = 0;
   for (uint32_t l = 0; l < nlev; l++) {
     const uint32_t n3[3] = {nx, ny, nz};
-    for (int a = 0; a < 3; a++) E[l][a] = l == 0 ? n3[a] : br.bd[l][a] * 128u;
+    uint32_t E[3];
+    for (int a = 0; a < 3; a++) E[a] = l == 0 ? n3[a] : br.bd[l][a] * 128u;
+    src[l] = {voxels, E[0], E[1], E[2], br.bd[l][0], br.bd[l][1], 0u};
     lev_off[l] = lev_total;
-    lev_total += ((size_t)E[l][0] * E[l][1] * E[l][2] + 255) & ~(size_t)255;
+    if (l || !dev_in) lev_total += ((size_t)E[0] * E[1] * E[2] + 255) & ~(size_t)255;
   }
   // resident bricks of every level and their slots, from the page table
   std::vector<uint32_t> page(c->page_words);
   R3D_CUDA_TRY(c, cudaMemcpy(page.data(), c->page, page.size() * 4, cudaMemcpyDeviceToHost));
-  std::vector<uint32_t> jobs_src, jobs_dst, lvl_count(nlev, 0);
+  std::vector<uint32_t> jobs_src, jobs_dst;
   for (uint32_t l = 0; l < nlev; l++) {
     const uint32_t nb = br.bd[l][0] * br.bd[l][1] * br.bd[l][2];
+    src[l].job0 = (uint32_t)jobs_src.size();
     for (uint32_t bi = 0; bi < nb; bi++) {
       const uint32_t e = page[br.off[l] + bi];
       if (e == R3D_BRICK_ABSENT || (e & 0xFFFFFFu) >= c->nslots) continue;
       jobs_src.push_back(bi);
       jobs_dst.push_back(e & 0xFFFFFFu);
-      lvl_count[l]++;
     }
   }
-  const size_t nj = jobs_src.size();
-  const size_t pool_bytes = (size_t)(c->nslots ? c->nslots : 1u) * (128u * 128u * 128u);
+  const size_t nj = jobs_src.size(), nslots = c->nslots ? c->nslots : 1u;
+  // the display filter works on slot bytes; without it the levels go
+  // straight to quad words
+  const bool filter = which < 2u && c->nslots && postfilter_on(c, which + 1u);
   uint8_t *lev = nullptr, *pool = nullptr;
-  uint32_t *jobs = nullptr;
-  cudaError_t e = cudaMalloc(&lev, lev_total);
-  if (e == cudaSuccess) e = cudaMalloc(&pool, pool_bytes);
-  if (e == cudaSuccess) e = cudaMalloc(&jobs, (nj ? nj : 1u) * 8);
-  if (e == cudaSuccess) e = cudaMemsetAsync(pool, 0, pool_bytes, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(lev, voxels, (size_t)nx * ny * nz, cudaMemcpyDefault, st);
+  uint32_t *jobs = nullptr, *quad = nullptr;
+  cudaError_t e = cudaMalloc(&lev, lev_total + (nj ? nj : 1u) * 8);
+  if (e == cudaSuccess) e = filter ? cudaMalloc(&pool, nslots * (128u * 128u * 128u))
+                                   : cudaMalloc(&quad, nslots * (128u * 128u * 128u) * 4u);
+  if (e == cudaSuccess && nj < c->nslots)  // slots that no brick of the table names
+    e = filter ? cudaMemsetAsync(pool, 0, nslots * (128u * 128u * 128u), st)
+               : cudaMemsetAsync(quad, 0, nslots * (128u * 128u * 128u) * 4u, st);
+  if (e == cudaSuccess && !dev_in) {
+    e = cudaMemcpyAsync(lev, voxels, (size_t)nx * ny * nz, cudaMemcpyDefault, st);
+    src[0].p = lev;
+  }
   for (uint32_t l = 1; l < nlev && e == cudaSuccess; l++) {
-    const size_t n = (size_t)E[l][0] * E[l][1] * E[l][2];
-    if (which == 2u)  // labels: stride sampling, never blended
-      k_label_stride<<<ovl_grid(n), 256, 0, st>>>(lev, nx, ny, nz, l, lev + lev_off[l], E[l][0],
-                                                   E[l][1], E[l][2]);
-    else  // the CT's (sum+4)/8 box pyramid
-      k_downsample_zero<<<ovl_grid(n), 256, 0, st>>>(lev + lev_off[l - 1], E[l - 1][0],
-                                                     E[l - 1][1], E[l - 1][2], lev + lev_off[l],
-                                                     E[l][0], E[l][1], E[l][2]);
-    e = cudaGetLastError();
+    const LevelSrc &p = src[l - 1];
+    uint8_t *dst = lev + lev_off[l];
+    if (which == 2u) {  // labels: stride sampling, never blended
+      const size_t n = (size_t)src[l].ex * src[l].ey * src[l].ez;
+      k_label_stride<<<ovl_grid(n), 256, 0, st>>>(src[0].p, nx, ny, nz, l, dst, src[l].ex,
+                                                   src[l].ey, src[l].ez);
+      e = cudaGetLastError();
+    } else {  // the CT's (sum+4)/8 box pyramid
+      e = launch_level_down(p.p, p.ex, p.ey, p.ez, dst, src[l].ex, src[l].ey, src[l].ez, nullptr,
+                            p.bdx, p.bdy, st);
+    }
+    src[l].p = dst;
   }
   if (e == cudaSuccess && nj) {
+    jobs = (uint32_t *)(lev + lev_total);
     e = cudaMemcpyAsync(jobs, jobs_src.data(), nj * 4, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(jobs + nj, jobs_dst.data(), nj * 4, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess)
+      e = launch_slot_fill(src, nlev, jobs, jobs + nj, (uint32_t)nj, pool, quad, nullptr, st);
   }
-  size_t joff = 0;
-  for (uint32_t l = 0; l < nlev && e == cudaSuccess; l++) {
-    for (uint32_t j0 = 0; j0 < lvl_count[l] && e == cudaSuccess; j0 += 65535u) {
-      const uint32_t n = min(lvl_count[l] - j0, 65535u);
-      k_brick_copy<<<dim3(128, n), 256, 0, st>>>(lev + lev_off[l], E[l][0], E[l][1], E[l][2],
-                                                 br.bd[l][0], br.bd[l][1], jobs + joff + j0,
-                                                 jobs + nj + joff + j0, pool);
-      e = cudaGetLastError();
-    }
-    joff += lvl_count[l];
+  int rc;
+  if (filter) {
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    rc = e == cudaSuccess ? set_overlay(c, which, pool, true) : cuda_fail(c, e, "bricks_overlay_build");
+  } else if (quad) {
+    rc = adopt_overlay(c, which, quad, e);
+  } else {
+    rc = cuda_fail(c, e, "bricks_overlay_build");
   }
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  int rc = e == cudaSuccess ? set_overlay(c, which, pool, true) : cuda_fail(c, e, "bricks_overlay_build");
   cudaFree(lev);
   cudaFree(pool);
-  cudaFree(jobs);
   return rc;
 }
 

@@ -10,6 +10,7 @@
 
 #include <vector>
 
+#include "r3d_build.cuh"
 #include "r3d_internal.h"
 
 namespace r3d {
@@ -75,8 +76,6 @@ __global__ void k_downsample_clamp(const uint8_t *__restrict__ src, uint32_t sx,
                                    uint32_t dy, uint32_t dz);
 __global__ void k_occ_dilate(const uint8_t *__restrict__ raw, uint8_t *__restrict__ dil,
                              uint32_t ox, uint32_t oy, uint32_t oz);
-__global__ void k_brick_max(const uint8_t *__restrict__ lev, uint32_t ex, uint32_t ey,
-                            uint32_t ez, uint32_t bdx, uint32_t bdy, uint32_t *__restrict__ out);
 
 static unsigned shard_grid(size_t n) {
   size_t b = (n + 255) / 256;
@@ -171,7 +170,11 @@ int r3d_cuda_shard_build(r3d_cuda_ctx *c, uint32_t edge, const uint8_t *voxels, 
         return frc;
       }
     }
-    k_brick_max<<<nb, 256, 0, c->stream>>>(vol, edge, edge, edge, bpa, bpa, dmax);
+    const uint32_t half = (bpa + 1u) / 2u * 128u;  // brick maxima of the volume itself
+    e = cudaMemsetAsync(dmax, 0, sizeof(uint32_t) * nb, c->stream);
+    if (e == cudaSuccess)
+      e = launch_level_down(vol, edge, edge, edge, nullptr, half, half, half, dmax, bpa, bpa,
+                            c->stream);
     for (uint32_t m = 1; m < 4u; m++) {
       const uint32_t s = a >> (m - 1), d = a >> m;
       k_downsample_clamp<<<shard_grid((size_t)d * d * d), 256, 0, c->stream>>>(
@@ -179,7 +182,7 @@ int r3d_cuda_shard_build(r3d_cuda_ctx *c, uint32_t edge, const uint8_t *voxels, 
     }
     k_shard_occ_raw<<<shard_grid(onb), 256, 0, c->stream>>>(buf, abpa, dslot, bpa, buf + total);
     k_occ_dilate<<<shard_grid(onb), 256, 0, c->stream>>>(buf + total, buf + off[4], od, od, od);
-    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaGetLastError();
   }
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(maxv.data(), dmax, sizeof(uint32_t) * nb, cudaMemcpyDeviceToHost,

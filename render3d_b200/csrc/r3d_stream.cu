@@ -15,41 +15,13 @@
 #include <algorithm>
 #include <vector>
 
+#include "r3d_build.cuh"
 #include "r3d_host.h"
 #include "r3d_internal.h"
 
 namespace r3d {
 
 constexpr uint32_t kSlotBytes = 128u * 128u * 128u;
-
-// Quad words and dilated 8^3 block maxima of the listed slots (the per-slot
-// tables of k_slot_quads / k_slot_blockmax).  Grid: (blocks, jobs).
-__global__ void k_stream_fill(const uint8_t *__restrict__ pool, const uint32_t *__restrict__ jobs,
-                              uint32_t *__restrict__ quad, uint8_t *__restrict__ bmax) {
-  const uint32_t s = jobs[blockIdx.y];
-  const uint8_t *g = pool + (size_t)s * kSlotBytes;
-  uint32_t *q = quad + (size_t)s * kSlotBytes;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < kSlotBytes;
-       i += gridDim.x * blockDim.x) {
-    const uint32_t x = i & 127u, y = (i >> 7) & 127u;
-    const uint32_t dx = x < 127u ? 1u : 0u, dy = y < 127u ? 128u : 0u;
-    q[i] = (uint32_t)g[i] | ((uint32_t)g[i + dx] << 8) | ((uint32_t)g[i + dy] << 16) |
-           ((uint32_t)g[i + dy + dx] << 24);
-  }
-  for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < 4096u;
-       e += gridDim.x * blockDim.x) {
-    const uint32_t bx = e & 15u, by = (e >> 4) & 15u, bz = e >> 8;
-    uint32_t m = 0;
-    for (uint32_t z = bz * 8u; z <= min(bz * 8u + 8u, 127u); z++)
-      for (uint32_t y = by * 8u; y <= min(by * 8u + 8u, 127u); y++) {
-        const uint8_t *row = g + ((size_t)z << 14) + ((size_t)y << 7);
-        for (uint32_t x = bx * 8u; x <= min(bx * 8u + 8u, 127u); x++)
-          m = max(m, (uint32_t)row[x]);
-      }
-    bmax[(size_t)s * 4096u + e] = (uint8_t)m;
-  }
-}
-
 
 // Copies the listed (slot, store index) bricks in, refills their tables and
 // publishes the page shadow.
@@ -67,8 +39,7 @@ static int stream_upload(r3d_cuda_ctx *c, const std::vector<uint32_t> &slots,
     const uint32_t nj = (uint32_t)std::min<size_t>(slots.size() - j0, 65535u);
     R3D_CUDA_TRY(c, cudaMemcpyAsync(c->stream_jobs + j0, slots.data() + j0, nj * 4u,
                                     cudaMemcpyHostToDevice, st));
-    k_stream_fill<<<dim3(64, nj), 256, 0, st>>>(c->pool, c->stream_jobs + j0, c->quad, c->bmax);
-    R3D_CUDA_TRY(c, cudaGetLastError());
+    R3D_CUDA_TRY(c, launch_slot_tables(c->pool, c->stream_jobs + j0, nj, c->quad, c->bmax, st));
     // the job list is reused by the next chunk: keep the kernel ahead of it
     if (j0 + nj < slots.size()) R3D_CUDA_TRY(c, cudaStreamSynchronize(st));
   }
@@ -132,18 +103,18 @@ int r3d_cuda_stream_begin(r3d_cuda_ctx *c, const r3d_volume_desc *d, const uint8
     return cuda_fail(c, e, "stream_begin: host store");
   }
   // the device pool shrinks to nslots slots, all empty
-  cudaFree(c->pool);
-  c->pool = nullptr;
-  e = cudaMalloc(&c->pool, (size_t)nslots * kSlotBytes);
-  if (e == cudaSuccess) e = cudaMemsetAsync(c->pool, 0, (size_t)nslots * kSlotBytes, c->stream);
-  if (e != cudaSuccess) {
+  rc = replace_pool(c, nslots);
+  if (rc == R3D_OK) {
+    e = cudaMemsetAsync(c->pool, 0, (size_t)nslots * kSlotBytes, c->stream);
+    if (e != cudaSuccess) rc = cuda_fail(c, e, "stream_begin: slot pool");
+  }
+  if (rc != R3D_OK) {
     stream_reset(c);
     c->have_bricks = false;
-    return cuda_fail(c, e, "stream_begin: slot pool");
+    return rc;
   }
   c->nslots = nslots;
   c->abpa = atlas_bpa(nslots);
-  c->br.pool = c->pool;
   c->br.nslots = nslots;
   rc = build_blockmax(c);
   if (rc != R3D_OK) {
