@@ -446,13 +446,13 @@ int r3d_cuda_raycast_fwd_noalloc(r3d_cuda_ctx *ctx, const r3d_frame_params *view
  * render, one thread per ray for one view (a batch resolves it once, from
  * its view count).  blocks_per_sm = resident
  * 128-thread blocks per SM of a persistent launch (0: the occupancy
- * limit).  shade_group (FULL mode, one-thread-per-ray launches):
- * n > 0 lets lanes park a sample that needs gradient shading until n lanes
- * of the warp (or all its live lanes) wait, and shades them together (1:
- * each sample where its ray meets it); 0 picks the sampling path's default,
- * 16 for the tiled slab, clipmap and virtual slab, whose gradient taps are
- * whole section lookups, and ungrouped shading for the cube and brick
- * paths.  Results are identical under every schedule. */
+ * limit).  shade_group (FULL mode, one-thread-per-ray launches): n > 0
+ * leaves samples that need gradient shading in a queue of the warp until n
+ * of them wait, and shades them together, one per lane (1: as soon as a step
+ * of the warp leaves any); 0 picks the sampling path's default: 32 on the
+ * cube, shard, tiled-slab, clipmap and virtual-slab paths, and shading where
+ * the ray meets the sample for LOD bricks.  Results are identical under every
+ * schedule. */
 typedef struct r3d_cuda_schedule {
   uint32_t persistent;
   uint32_t refill_min;

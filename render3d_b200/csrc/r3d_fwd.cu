@@ -24,7 +24,7 @@
 #define R3D_FWD_BOUNDS                                                                     \
   __launch_bounds__(R3D_FWD_WARPS * 32,                                                    \
                     (R3D_FWD_MIN_BLOCKS + (PATH == PATH_LOD_BRICKS && !OVL && !COUNT &&    \
-                                                   !DEFER && MODE != R3D_MODE_HEATMAP            \
+                                                   !QUEUE && MODE != R3D_MODE_HEATMAP            \
                                                ? (MODE == R3D_MODE_MIP ? 2 : 1)                  \
                                                : 0)) * 4 / R3D_FWD_WARPS)
 #else
@@ -38,13 +38,9 @@ constexpr uint32_t kBlockW = kFwdWarps >= 2 ? 16u : 8u;  // dispatch threads per
 constexpr uint32_t kBlockH = kFwdWarps == 4 ? 8u : 4u;   // and y
 static_assert(kFwdWarps == 1 || kFwdWarps == 2 || kFwdWarps == 4, "1, 2 or 4 warps");
 
-// DEFER (FULL mode): gradient shading is the long branch of a step and
-// usually only one or two lanes of a warp need it at once.  A lane that
-// reaches a shaded sample parks it (ray_step returns kStepShade); the warp
-// shades the parked samples together once at least shade_min lanes are
-// waiting or every live lane is, so the branch runs with more lanes active.
-// Rays are independent, so each ray's arithmetic and result are unchanged.
-template <int PATH, int MODE, bool FAST, bool COUNT, bool DEFER, bool OVL = false>
+// QUEUE (FULL mode): contributing samples are shaded through the warp's
+// shading queue (ShadeQueue), group at a time.
+template <int PATH, int MODE, bool FAST, bool COUNT, bool QUEUE, bool OVL = false>
 __global__ void R3D_FWD_BOUNDS k_raycast(const __grid_constant__ r3d_frame_params pc,
                                          const __grid_constant__ DevScene s,
                                          const uchar4 *__restrict__ lut,
@@ -53,8 +49,9 @@ __global__ void R3D_FWD_BOUNDS k_raycast(const __grid_constant__ r3d_frame_param
                                          uint32_t *__restrict__ mip_out,
                                          unsigned long long *__restrict__ total,
                                          unsigned long long *__restrict__ counters,
-                                         uint32_t shade_min, uint32_t row0) {
+                                         uint32_t group, uint32_t row0) {
   __shared__ float4 tf[256];
+  __shared__ ShadeQueue sq[QUEUE ? kFwdWarps : 1u];
   for (uint32_t i = threadIdx.x; i < 256u; i += blockDim.x) {
     uchar4 u = lut[i];
     tf[i] = make_float4((float)u.x, (float)u.y, (float)u.z, (float)u.w);
@@ -112,36 +109,10 @@ __global__ void R3D_FWD_BOUNDS k_raycast(const __grid_constant__ r3d_frame_param
   const bool inside = px < vw && py < vh;
   const ViewConst vc = view_const<PATH>(pc, s);
   RayResult r;
-  if (DEFER) {
-    RayState st;
-    Pending pend;
-    bool active = inside && ray_begin<PATH, MODE>(pc, s, vc, px, py, st, r);
-    const bool marched = active;
-    bool parked = false;
-    while (true) {
-      if (__ballot_sync(0xffffffffu, active) == 0u) break;
-      if (active && !parked) {
-        const int rs = ray_step<PATH, MODE, FAST, COUNT, true>(s, vc, tf, st, pend);
-        if (rs == kStepDone)
-          active = false;
-        else if (rs == kStepShade)
-          parked = true;
-      }
-      const uint32_t need = __ballot_sync(0xffffffffu, parked);
-      if (need != 0u) {
-        const uint32_t live = __ballot_sync(0xffffffffu, active);
-        if ((uint32_t)__popc(need) >= shade_min || need == live) {
-          if (parked) {
-            parked = false;
-            if (!composite_sample<PATH, MODE, FAST, COUNT>(s, vc, st, pend)) active = false;
-          }
-        }
-      }
-    }
-    if (marched) ray_end<MODE>(vc, st, r);
-  } else {
+  if constexpr (QUEUE)
+    march_queued<PATH, MODE, FAST, COUNT>(pc, s, vc, tf, px, py, inside, r, sq[warp], group);
+  else
     march_warp<PATH, MODE, FAST, COUNT, OVL>(pc, s, vc, tf, px, py, inside, r);
-  }
   if (inside) {
     my_tf = r.n_tf;
     my_grad = r.n_grad;
@@ -189,7 +160,9 @@ static cudaError_t launch_t(const r3d_frame_params &pc, const DevScene &s, const
   if (row0 >= row1) return cudaSuccess;
   dim3 grid((gw + kBlockW - 1u) / kBlockW, (row1 - row0 + kBlockH - 1u) / kBlockH);
   const uint32_t threads = kFwdWarps * 32u;
-  constexpr bool kDeferable = MODE == R3D_MODE_FULL;
+  // FULL views with and without the queue: LOD bricks (by the schedule); the
+  // other paths' FULL views always queue
+  constexpr bool kQueue = MODE == R3D_MODE_FULL, kDirect = !kQueue || !kShadeQueued<PATH, MODE, false>;
   // overlay atlases: LOD bricks in the compositing and MIP modes
   constexpr bool kOvl = PATH == PATH_LOD_BRICKS &&
                         (MODE == R3D_MODE_FULL || MODE == R3D_MODE_FLAT || MODE == R3D_MODE_MIP);
@@ -204,19 +177,25 @@ static cudaError_t launch_t(const r3d_frame_params &pc, const DevScene &s, const
       return cudaGetLastError();
     }
   }
-  if (kDeferable && shade) {
+  if constexpr (kQueue) {
+    if (shade || !kDirect) {
+      if (!shade) shade = 32u;
+      if (counters)
+        k_raycast<PATH, MODE, FAST, true, true><<<grid, threads, 0, stream>>>(
+            pc, s, lut, (uchar4 *)img, out_w, steps, mip, total, counters, shade, row0);
+      else
+        k_raycast<PATH, MODE, FAST, false, true><<<grid, threads, 0, stream>>>(
+            pc, s, lut, (uchar4 *)img, out_w, steps, mip, total, nullptr, shade, row0);
+      return cudaGetLastError();
+    }
+  }
+  if constexpr (kDirect) {
     if (counters)
-      k_raycast<PATH, MODE, FAST, true, kDeferable><<<grid, threads, 0, stream>>>(
-          pc, s, lut, (uchar4 *)img, out_w, steps, mip, total, counters, shade, row0);
+      k_raycast<PATH, MODE, FAST, true, false><<<grid, threads, 0, stream>>>(
+          pc, s, lut, (uchar4 *)img, out_w, steps, mip, total, counters, 0u, row0);
     else
-      k_raycast<PATH, MODE, FAST, false, kDeferable><<<grid, threads, 0, stream>>>(
-          pc, s, lut, (uchar4 *)img, out_w, steps, mip, total, nullptr, shade, row0);
-  } else if (counters) {
-    k_raycast<PATH, MODE, FAST, true, false><<<grid, threads, 0, stream>>>(
-        pc, s, lut, (uchar4 *)img, out_w, steps, mip, total, counters, 0u, row0);
-  } else {
-    k_raycast<PATH, MODE, FAST, false, false><<<grid, threads, 0, stream>>>(
-        pc, s, lut, (uchar4 *)img, out_w, steps, mip, total, nullptr, 0u, row0);
+      k_raycast<PATH, MODE, FAST, false, false><<<grid, threads, 0, stream>>>(
+          pc, s, lut, (uchar4 *)img, out_w, steps, mip, total, nullptr, 0u, row0);
   }
   return cudaGetLastError();
 }
@@ -282,14 +261,8 @@ cudaError_t launch_view(const r3d_cuda_ctx *c, const r3d_frame_params &pc, uint8
   DevScene s = c->scene();
   s.el = elide_counts(pc, s.tf_zero_t);
   const bool fast = c->quality == R3D_QUALITY_FAST;
-  // shade_group 0 picks the path's default: grouped shading pays where a
-  // gradient tap is a whole section lookup (tiled slab, clipmap, virtual
-  // slab: 13-31 % faster frames at 16) and costs where it is a fetch inside
-  // the cached brick (LOD bricks, cube: 1.7x slower frames)
   const int path = path_of_view(pc);
-  const uint32_t shade = c->sched.shade_group ? c->sched.shade_group
-                         : (path == PATH_SLAB || path == PATH_CLIP || path == PATH_VSLAB) ? 16u
-                                                                                          : 0u;
+  const uint32_t shade = c->sched.shade_group;  // 0: the path's default (kShadeQueued)
 #define R3D_PATH_CASE(P)                                                                   \
   case P:                                                                                  \
     return launch_path<P>(pc, s, fast, c->lut, img, out_w, steps, mip_index, total, counters, \

@@ -870,12 +870,17 @@ __device__ __forceinline__ ViewConst view_const(const r3d_frame_params &pc, cons
   return view_const<PATH>(pc, s, s.el);
 }
 
-enum { kStepDone = 0, kStepCont = 1, kStepShade = 2 };
+// kStepShade and kStepLast: a contributing sample was left for shading (the
+// ray goes on, or ends with it)
+enum { kStepDone = 0, kStepCont = 1, kStepShade = 2, kStepLast = 3 };
 
-// A contributing sample waiting for gradient shading and compositing.
+// A contributing sample: what its colour, and its weight in the ray's sums,
+// depend on.
 struct Pending {
   float3 p;
-  float lod, lod_step, a;
+  float lod, lod_step;
+  float a;    // opacity; of a sample left for shading: its weight, (1 - accumulated) * opacity
+  float tt;   // TF coordinate
   float4 sm;  // TF sample
   uint32_t slot;
   float3 bl;
@@ -1062,13 +1067,12 @@ __device__ __forceinline__ float tap_sample(const DevScene &s, const DevCube &te
 
 // Colour of a contributing sample: the TF colour, gradient shading (FULL
 // mode, raycast.slang:919-998) and the overlay tints (:1000-1014).
-template <int PATH, int MODE, bool FAST, bool COUNT, bool OVL = false>
-__device__ __forceinline__ float3 sample_color(const DevScene &s, const ViewConst &vc,
-                                               RayState &st, const Pending &q) {
+template <int PATH, int MODE, bool FAST, bool OVL = false>
+__device__ __forceinline__ float3 sample_color(const DevScene &s, const ViewConst &vc, float3 dir,
+                                               const Pending &q) {
   constexpr bool kLod = PATH == PATH_LOD_BRICKS;
   constexpr bool kShard = PATH == PATH_SHARD;
   constexpr bool kShaded = MODE == R3D_MODE_FULL;
-  const float3 dir = st.dir;
   float col_r = q.sm.x, col_g = q.sm.y, col_b = q.sm.z;
   if (OVL && q.reg_live) {  // green/magenta fuse in TF space, before shading (:910-914)
     const float3 wl = make_float3(0.333f, 0.334f, 0.333f);
@@ -1086,7 +1090,6 @@ __device__ __forceinline__ float3 sample_color(const DevScene &s, const ViewCons
   const bool slot_taps = kShard && !s.sh.identity;
   constexpr bool kSection = PATH == PATH_SLAB || PATH == PATH_CLIP || PATH == PATH_VSLAB;
   if (kShaded) {
-    if (COUNT) st.n_grad++;
     float g0, g1, g2;
     if (FAST) {  // raycast.slang:919-955
       const float ir3 = 0.57735026919f, renorm = 0.86602540378f;
@@ -1264,13 +1267,13 @@ __device__ __forceinline__ float3 sample_color(const DevScene &s, const ViewCons
   return make_float3(col_r, col_g, col_b);
 }
 
-// Gradient shading and front-to-back compositing (raycast.slang:1015-1017)
-// of a contributing sample, then the step advance (:1020).  Returns false
-// when the opacity cutoff ends the ray.
-template <int PATH, int MODE, bool FAST, bool COUNT, bool OVL = false>
+// Colour and front-to-back compositing (raycast.slang:1015-1017) of a
+// contributing sample, then the step advance (:1020).  Returns false when
+// the opacity cutoff ends the ray.
+template <int PATH, int MODE, bool FAST, bool OVL = false>
 __device__ __forceinline__ bool composite_sample(const DevScene &s, const ViewConst &vc,
                                                  RayState &st, const Pending &q) {
-  const float3 col = sample_color<PATH, MODE, FAST, COUNT, OVL>(s, vc, st, q);
+  const float3 col = sample_color<PATH, MODE, FAST, OVL>(s, vc, st.dir, q);
   float wgt = (1.0f - st.acc_a) * q.a;
   st.acc_r = fmaf(wgt, col.x, st.acc_r);
   st.acc_g = fmaf(wgt, col.y, st.acc_g);
@@ -1279,48 +1282,6 @@ __device__ __forceinline__ bool composite_sample(const DevScene &s, const ViewCo
   if (st.acc_a >= s.alpha_cutoff) return false;
   st.t = fmaf(vc.dt, q.lod_step, st.t);
   return true;
-}
-
-// Shading later (LOD bricks, FULL mode).  The opacity a ray accumulates, and
-// so its termination and step positions, never depend on sample colours:
-// only the colour sums do, through rgb <- fma(w_i, c_i, rgb) in sample
-// order.  So the march can keep, for each contributing sample, its weight
-// w_i = (1 - A) a, its TF coordinate and its brick position, and leave the
-// shading (six brick taps, normal, lighting) for later.  A warp shades the
-// kept samples of all its rays together once every ray has ended, instead
-// of one or two lanes at a time inside divergent steps, and folds them into
-// the sums in the same order with the same operations: the image is
-// bit-identical.  A ray that keeps kShadeCap samples shades them at once.
-#ifndef R3D_SHADE_CAP
-#define R3D_SHADE_CAP 4
-#endif
-constexpr uint32_t kShadeCap = R3D_SHADE_CAP;
-struct ShadeEntry {
-  float wgt, tt, bx, by, bz, grad_vox;
-  uint32_t slot;
-};
-struct ShadeBuf {
-  ShadeEntry e[kShadeCap];
-  uint32_t n;
-};
-
-template <int PATH, int MODE, bool FAST, bool COUNT>
-__device__ __forceinline__ void shade_flush(const DevScene &s, const ViewConst &vc,
-                                            const float4 *tf, RayState &st, ShadeBuf &sb) {
-#pragma unroll 1
-  for (uint32_t k = 0; k < sb.n; k++) {
-    const ShadeEntry e = sb.e[k];
-    Pending q;
-    q.sm = tf_sample(tf, e.tt);
-    q.slot = e.slot;
-    q.bl = make_float3(e.bx, e.by, e.bz);
-    q.grad_vox = e.grad_vox;
-    const float3 col = sample_color<PATH, MODE, FAST, COUNT>(s, vc, st, q);
-    st.acc_r = fmaf(e.wgt, col.x, st.acc_r);
-    st.acc_g = fmaf(e.wgt, col.y, st.acc_g);
-    st.acc_b = fmaf(e.wgt, col.z, st.acc_b);
-  }
-  sb.n = 0;
 }
 
 // The footprint ratio of a sample at t (raycast.slang:772-774).
@@ -1366,14 +1327,14 @@ __device__ __forceinline__ void lod_range(RayState &st, const ViewConst &vc, int
 
 // One iteration of the hot loop (raycast.slang:767-1021).  Returns
 // kStepDone when the ray is finished (loop condition failed, saturation or
-// opacity cutoff) and kStepCont otherwise.  With DEFER, a sample that needs
-// gradient shading stops before it: the sample is left in pend and
-// kStepShade returned; composite_sample(pend) completes the iteration.
+// opacity cutoff) and kStepCont otherwise.  With DEFER, the colour of a
+// contributing sample is left out: the sample stands in pend, its weight is
+// in the accumulated opacity and the ray has moved on (kStepShade) or ended
+// (kStepLast).
 template <int PATH, int MODE, bool FAST, bool COUNT, bool DEFER = false, bool OVL = false,
-          bool LATER = false, bool STAGE = false>
+          bool STAGE = false>
 __device__ __forceinline__ int ray_step(const DevScene &s, const ViewConst &vc, const float4 *tf,
-                                        RayState &st, Pending &pend, ShadeBuf *sb = nullptr,
-                                        const StageBox *box = nullptr) {
+                                        RayState &st, Pending &pend, const StageBox *box = nullptr) {
   constexpr bool kLod = PATH == PATH_LOD_BRICKS;
   constexpr bool kShard = PATH == PATH_SHARD;
   constexpr bool kSlab = PATH == PATH_SLAB;
@@ -1581,23 +1542,19 @@ __device__ __forceinline__ int ray_step(const DevScene &s, const ViewConst &vc, 
         sm.w = fmaxf(sm.w, rs.w * vc.reg_alpha);
       }
       float a = 1.0f - r3d_powf(1.0f - sm.w, vc.opac_k * lod_step);
-      if (LATER && a > 0.003f) {  // keep the sample; its colour comes later
-        const float wgt = (1.0f - st.acc_a) * a;
-        st.acc_a = st.acc_a + wgt;
-        sb->e[sb->n] = {wgt, tt, b.bl.x, b.bl.y, b.bl.z, b.grad_vox, b.slot};
-        if (++sb->n == kShadeCap) shade_flush<PATH, MODE, FAST, COUNT>(s, vc, tf, st, *sb);
-        if (st.acc_a >= s.alpha_cutoff) return kStepDone;
-        st.t = fmaf(vc.dt, lod_step, t);
-        return kStepCont;
-      }
       if (a > 0.003f) {
-        const Pending q = {p, lod, lod_step, a, sm, b.slot, b.bl, b.grad_vox, rs, reg_live};
-        if (DEFER && kShaded) {  // shading runs later, grouped across the warp
+        if (COUNT && kShaded) st.n_grad++;
+        const Pending q = {p, lod, lod_step, a, tt, sm, b.slot, b.bl, b.grad_vox, rs, reg_live};
+        if (DEFER) {
           pend = q;
+          const float wgt = (1.0f - st.acc_a) * a;
+          pend.a = wgt;
+          st.acc_a = st.acc_a + wgt;
+          if (st.acc_a >= s.alpha_cutoff) return kStepLast;
+          st.t = fmaf(vc.dt, lod_step, st.t);
           return kStepShade;
         }
-        return composite_sample<PATH, MODE, FAST, COUNT, OVL>(s, vc, st, q) ? kStepCont
-                                                                           : kStepDone;
+        return composite_sample<PATH, MODE, FAST, OVL>(s, vc, st, q) ? kStepCont : kStepDone;
       }
     }
   }
@@ -1677,39 +1634,129 @@ __device__ __forceinline__ void march(const r3d_frame_params &pc, const DevScene
   ray_end<MODE, OVL>(vc, st, out);
 }
 
-// Whether a kernel instantiation shades later (see shade_flush).
-#ifndef R3D_SHADE_LATER
-#define R3D_SHADE_LATER 0
-#endif
-template <int PATH, int MODE, bool OVL>
-constexpr bool kShadesLater =
-    R3D_SHADE_LATER && PATH == PATH_LOD_BRICKS && MODE == R3D_MODE_FULL && !OVL;
-
-// march() for every lane of a warp (all 32 lanes call it; `inside` says
-// whether the lane has a ray): with shading later, the rays march, the warp
-// reconverges, and the kept samples of all its rays are shaded together.
+// march() of a warp's lanes that have a ray.  (Called through this wrapper the
+// whole-tile kernel's LOD-brick FULL views fit their 64 registers; with the
+// branch written out in the kernel they spill 60 bytes and lose 3 %.)
 template <int PATH, int MODE, bool FAST, bool COUNT = false, bool OVL = false>
 __device__ __forceinline__ void march_warp(const r3d_frame_params &pc, const DevScene &s,
                                            const ViewConst &vc, const float4 *tf, uint32_t px,
                                            uint32_t py, bool inside, RayResult &out) {
-  if constexpr (kShadesLater<PATH, MODE, OVL>) {
-    RayState st;
-    Pending pend;
-    ShadeBuf sb;
-    sb.n = 0;
-    const bool marched = inside && ray_begin<PATH, MODE>(pc, s, vc, px, py, st, out);
-    if (marched)
-      while (ray_step<PATH, MODE, FAST, COUNT, false, false, true>(s, vc, tf, st, pend, &sb) !=
-             kStepDone) {
-      }
-    __syncwarp();
-    if (marched) {
-      shade_flush<PATH, MODE, FAST, COUNT>(s, vc, tf, st, sb);
-      ray_end<MODE>(vc, st, out);
-    }
-  } else {
-    if (inside) march<PATH, MODE, FAST, COUNT, OVL>(pc, s, vc, tf, px, py, out);
+  if (inside) march<PATH, MODE, FAST, COUNT, OVL>(pc, s, vc, tf, px, py, out);
+}
+
+// The shading queue of one warp (FULL mode).  The opacity a ray accumulates,
+// and so its step positions and its end, never depends on sample colours:
+// only the colour sums do, through rgb <- fma(w_i, c_i, rgb) in sample order.
+// So the march leaves each contributing sample in the queue -- its weight
+// w_i, its TF coordinate and where it lies -- and goes on; whenever a warp's
+// worth is waiting, every lane shades one of them, whichever ray it belongs
+// to, and each ray then folds its own into its sums, oldest first: the same
+// operations in the same order, so the image is bit-identical.  Shading is
+// the longest branch of a step (six or four gradient taps) and one or two
+// lanes of a divergent warp reach it at a time.
+struct ShadeQueue {
+  float4 a[64];      // where: p (cube-like paths) or the brick position, and tt; then the colour
+  float4 b[64];      // lod (LOD bricks: grad_vox), lod_step, weight, ray | slot << 5
+  uint32_t own[32];  // per ray: its entries of the batch
+};
+
+// Shades the n <= 32 oldest entries (from head), all lanes together.
+template <int PATH, int MODE, bool FAST>
+__device__ __forceinline__ void shade_batch(const DevScene &s, const ViewConst &vc,
+                                            const float4 *tf, RayState &st, ShadeQueue &q,
+                                            uint32_t head, uint32_t n) {
+  constexpr uint32_t kAll = 0xffffffffu;
+  const uint32_t lane = threadIdx.x & 31u, e = (head + lane) & 63u;
+  const bool mine = lane < n;
+  const float4 A = q.a[e], B = q.b[e];
+  const uint32_t tag = __float_as_uint(B.w), ray = tag & 31u;
+  const float3 dir = make_float3(__shfl_sync(kAll, st.dir.x, ray), __shfl_sync(kAll, st.dir.y, ray),
+                                 __shfl_sync(kAll, st.dir.z, ray));
+  q.own[lane] = 0u;
+  const uint32_t peers = __match_any_sync(kAll, mine ? ray : 32u + lane);
+  if (mine) {
+    Pending p;
+    p.p = p.bl = make_float3(A.x, A.y, A.z);
+    p.lod = p.grad_vox = B.x;
+    p.lod_step = B.y;
+    p.slot = (uint32_t)((int)tag >> 5);  // signed: a clip level may be -1
+    p.sm = tf_sample(tf, A.w);
+    p.reg_live = false;
+    const float3 c = sample_color<PATH, MODE, FAST>(s, vc, dir, p);
+    q.a[e] = make_float4(c.x, c.y, c.z, B.z);
   }
+  __syncwarp();
+  if (mine) q.own[ray] = peers;
+  __syncwarp();
+  for (uint32_t m = q.own[lane]; m; m &= m - 1u) {
+    const float4 c = q.a[(head + (uint32_t)__ffs((int)m) - 1u) & 63u];
+    st.acc_r = fmaf(c.w, c.x, st.acc_r);
+    st.acc_g = fmaf(c.w, c.y, st.acc_g);
+    st.acc_b = fmaf(c.w, c.z, st.acc_b);
+  }
+  __syncwarp();
+}
+
+// Whether a kernel's FULL views shade through the queue when the schedule
+// does not say (shade_group 0).  Measured on whole frames, queue against
+// shading in place (sections: against parking 16 lanes' samples): tiled slab
+// 2.74 -> 1.79 ms (3.8 shaded samples a pixel), virtual slab 2.13 -> 1.35,
+// 512^3 shard 1.84 -> 1.74, 256^3 cube 0.58 -> 0.57, a thumbnail 0.23 -> 0.17;
+// LOD bricks lose (1080p frame 0.507 -> 0.540, four panes 0.60 -> 0.67): a
+// tap there is two loads in the cached brick, and the votes of every step
+// cost more than the idle lanes.
+template <int PATH, int MODE, bool OVL>
+constexpr bool kShadeQueued = MODE == R3D_MODE_FULL && !OVL && PATH != PATH_LOD_BRICKS;
+
+// march() for every lane of a warp (all 32 lanes call it; `inside` says
+// whether the lane has a ray) with the shading queue: `group` waiting samples
+// (1..32) start a batch.
+template <int PATH, int MODE, bool FAST, bool COUNT = false>
+__device__ __forceinline__ void march_queued(const r3d_frame_params &pc, const DevScene &s,
+                                             const ViewConst &vc, const float4 *tf, uint32_t px,
+                                             uint32_t py, bool inside, RayResult &out,
+                                             ShadeQueue &q, uint32_t group) {
+  constexpr uint32_t kAll = 0xffffffffu;
+  const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+  RayState st;
+  st.dir = make_float3(0.0f, 0.0f, 0.0f);
+  bool active = inside && ray_begin<PATH, MODE>(pc, s, vc, px, py, st, out);
+  const bool marched = active;
+  uint32_t head = 0, n = 0;  // the waiting entries: [head, head + n), mod 64
+  while (__any_sync(kAll, active)) {
+    Pending pend;
+    int r = kStepCont;
+    if (active) {
+      r = ray_step<PATH, MODE, FAST, COUNT, true>(s, vc, tf, st, pend);
+      active = r == kStepCont || r == kStepShade;
+    }
+    const uint32_t add = __ballot_sync(kAll, r >= kStepShade);
+    if (add) {
+      if (r >= kStepShade) {
+        const uint32_t e = (head + n + (uint32_t)__popc(add & below)) & 63u;
+        const bool in_slot = PATH == PATH_LOD_BRICKS || (PATH == PATH_SHARD && !s.sh.identity);
+        const float3 at = in_slot ? pend.bl : pend.p;
+        q.a[e] = make_float4(at.x, at.y, at.z, pend.tt);
+        q.b[e] = make_float4(PATH == PATH_LOD_BRICKS ? pend.grad_vox : pend.lod, pend.lod_step,
+                             pend.a, __uint_as_float(lane | (pend.slot << 5)));
+      }
+      n += (uint32_t)__popc(add);
+      __syncwarp();
+      if (n >= group) {
+        const uint32_t k = min(n, 32u);
+        shade_batch<PATH, MODE, FAST>(s, vc, tf, st, q, head, k);
+        head += k;
+        n -= k;
+      }
+    }
+  }
+  while (n) {
+    const uint32_t k = min(n, 32u);
+    shade_batch<PATH, MODE, FAST>(s, vc, tf, st, q, head, k);
+    head += k;
+    n -= k;
+  }
+  if (marched) ray_end<MODE>(vc, st, out);
 }
 
 }  // namespace r3d

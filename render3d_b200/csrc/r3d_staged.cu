@@ -130,9 +130,6 @@ __global__ void __launch_bounds__(kStageThreads, 16)
   RayResult r;
   RayState st;
   Pending pend;
-  ShadeBuf sbuf;
-  sbuf.n = 0;
-  constexpr bool kLater = MODE == R3D_MODE_FULL && R3D_SHADE_LATER;
   bool active = inside && ray_begin<PATH_LOD_BRICKS, MODE>(pc, s, vc, px, py, st, r);
   const bool marched = active;
   uint32_t phase = 0;
@@ -175,15 +172,12 @@ __global__ void __launch_bounds__(kStageThreads, 16)
     }
     if (active) {
       const StageBox sb = {box, sh_slot, sh_bx, sh_by, sh_bz};
-      if (ray_step<PATH_LOD_BRICKS, MODE, FAST, false, false, false, kLater, true>(
-              s, vc, tf, st, pend, &sbuf, &sb) == kStepDone)
+      if (ray_step<PATH_LOD_BRICKS, MODE, FAST, false, false, false, true>(s, vc, tf, st, pend,
+                                                                           &sb) == kStepDone)
         active = false;
     }
   }
-  if (marched) {
-    if (kLater) shade_flush<PATH_LOD_BRICKS, MODE, FAST, false>(s, vc, tf, st, sbuf);
-    ray_end<MODE>(vc, st, r);
-  }
+  if (marched) ray_end<MODE>(vc, st, r);
   uint32_t my_steps = 0;
   if (inside) {
     const uchar4 col = make_uchar4(unorm8(r.rgb[0]), unorm8(r.rgb[1]), unorm8(r.rgb[2]), 255);
