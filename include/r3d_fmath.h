@@ -130,4 +130,17 @@ R3D_FM_HD float r3d_powi24f(float x) {
   return x12 * x12;
 }
 
+/* a / b, correctly rounded, for a whole number 1 <= b < 2^20 with rb = 1 / b
+ * (rounded): a quotient estimate, its exact residual, and one correction
+ * (Markstein's division, IBM J. Res. Dev. 34(1), 1990).  The estimate lies
+ * within 2 ulp, so the residual is a multiple of ulp(q) below 2^21 times it
+ * and exact; and the quotient of a float by such a b is at least 2^-21 ulp
+ * away from every rounding boundary, above the error before the last
+ * rounding.  a is finite, and not so small that the quotient is subnormal
+ * (it may then be an ulp off). */
+R3D_FM_HD float r3d_div_by(float a, float b, float rb) {
+  float q = a * rb;
+  return fmaf(fmaf(-b, q, a), rb, q);
+}
+
 #endif /* R3D_FMATH_H */

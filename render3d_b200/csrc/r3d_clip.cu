@@ -152,6 +152,7 @@ int r3d_cuda_clip_build(r3d_cuda_ctx *c, const r3d_volume_desc *d, const uint8_t
   for (int l = 0; l < kClipLevels; l++) {
     cl.lev[l] = c->clip_tex + off;
     off += (size_t)kClipTex * kClipTex * cl.wzl[l];
+    cl.rwzl[l] = 1.0f / (float)cl.wzl[l];
     c->clip_layer[l].assign(cl.wzl[l], -1);
     c->clip_org[l][0] = c->clip_org[l][1] = INT64_MIN;  // not centred yet
   }

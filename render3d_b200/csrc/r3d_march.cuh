@@ -119,11 +119,15 @@ struct DevSlab {
   uint32_t ovs;       // overview downscale of the coarsest level
   float nx, ny, px, py, z0;  // the frame parameters slab_nx/ny/px/py/z0 of the window
   DevSlabLevel lev[kSlabLevels];
-  // per-view constants of vs_sample's overview branch (raycast.slang:430-446),
-  // evaluated once with the shader's own float expressions: the number of
-  // overview levels, and per level k the grid and payload gxl, gyl, pxl, pyl
-  int nov;
-  float ov[kSlabLevels][4];
+  // constants of slab_axis per level and axis, evaluated once: overview levels
+  // with the shader's own float expressions (raycast.slang:430-446)
+  int nov;       // overview levels a view may pick
+  float rwz;     // 1 / wz
+  struct Axis {  // (whole numbers)
+    float p, rp;  // payload, its reciprocal
+    float t, rt;  // p + 2, its reciprocal
+    float gmax;   // tiles - 1
+  } ax[kSlabLevels][2];
 };
 
 // XY clipmap (raycast.slang:357-408, src/core/clip.h): 6 nested levels of
@@ -135,6 +139,7 @@ struct DevClip {
   const uint8_t *lev[kClipLevels];
   uint32_t wzl[kClipLevels];
   float ox[kClipLevels], oy[kClipLevels];  // clip_orig of the frame parameters
+  float rwzl[kClipLevels];                 // 1 / wzl
   uint32_t valid;                          // clip_valid
   float nx, z0;                            // slab_nx, slab_z0
 };
@@ -154,6 +159,8 @@ struct DevVslab {
   uint32_t px, wz;
   uint32_t gx[kVsLevels], gy[kVsLevels], base[kVsLevels];
   float x0, y0, z0, nx;  // the frame parameters slab_x0/y0/z0 and slab_nx (= W)
+  float rp, rt, rwz;                             // reciprocals of px, px + 2, wz
+  float rg[kVsLevels][2];                        // and of gx, gy
 };
 
 // Byte-valued thresholds of the fetch elision.  A block maximum m (a byte)
@@ -619,51 +626,122 @@ __device__ __forceinline__ float shard_fetch(const DevShard &h, float3 org, floa
   return cube_sample(h.atlas, u, lod);
 }
 
-// A slab tile sampled at normalized (u, v, w) like the slab sampler
-// (src/vk/vkbackend.c:2203-2211): linear, clamp to edge in x and y (the
-// apron makes tiles seamless), REPEAT in w so the z ring wraps.
-__device__ __forceinline__ float tex_wrapz(const uint8_t *__restrict__ g, uint32_t tw, uint32_t th,
-                                           uint32_t wz, float u, float v, float w) {
-  const float tx = clamp_(fmaf(u, (float)tw, -0.5f), 0.0f, (float)(tw - 1u));
-  const float ty = clamp_(fmaf(v, (float)th, -0.5f), 0.0f, (float)(th - 1u));
-  const float tz = fmaf(w, (float)wz, -0.5f);
-  float fx, fy;
-  const uint32_t x0 = floor_frac(tx, fx), y0 = floor_frac(ty, fy);
-  const float zf = floorf(tz), fz = tz - zf;
-  // w is a fraction in [0, 1), so floor(tz) lies in [-1, wz - 1] and its
-  // ring layer is one conditional away (the modulo of the restatement)
-  const int zi = (int)zf;
-  const uint32_t z0 = zi < 0 ? wz - 1u : min((uint32_t)zi, wz - 1u);
-  const uint32_t z1 = z0 + 1u < wz ? z0 + 1u : 0u;
-  const uint32_t x1 = min(x0 + 1u, tw - 1u), y1 = min(y0 + 1u, th - 1u);
-  const size_t sy = tw, sz = (size_t)tw * th;
-  const uint8_t *r00 = g + y0 * sy + z0 * sz, *r10 = g + y1 * sy + z0 * sz;
-  const uint8_t *r01 = g + y0 * sy + z1 * sz, *r11 = g + y1 * sy + z1 * sz;
-  const float c00 = lerp_raw(raw_u8(r00 + x0), raw_u8(r00 + x1), fx);
-  const float c10 = lerp_raw(raw_u8(r10 + x0), raw_u8(r10 + x1), fx);
-  const float c01 = lerp_raw(raw_u8(r01 + x0), raw_u8(r01 + x1), fx);
-  const float c11 = lerp_raw(raw_u8(r11 + x0), raw_u8(r11 + x1), fx);
-  return lerp_(lerp_(c00, c10, fy), lerp_(c01, c11, fy), fz) * kInv255;
+// The lookups of the section paths (tiled slab, virtual slab, clipmap) are
+// separable: each axis of a position decides its tile, base texel and
+// fraction by itself, and a gradient tap moves one axis (or, of the four-tap
+// pattern, reuses two values per axis).  So a lookup is three axes and a
+// fetch, the taps of a sample share axes with each other and the sample, and
+// an axis divides by its whole-number sizes with r3d_div_by.  The frames are
+// bound by issue: whole lookups per tap with IEEE divisions took 1.79 ms
+// (tiled slab, 1080p FULL; FLAT 1.03) and 1.35 ms (virtual slab, 1600x900;
+// FLAT 0.77), this takes 1.33 (0.78) and 1.15 (0.64).
+
+// x or y: tile coordinate q of the sampled level, base texel i0 in the tile,
+// step d to its clamped neighbour, fraction; virtual slab: position b of the
+// base cell in its grid and the cell's key bits.
+struct SecAxis {
+  float q, f, b;
+  uint32_t i0, d, key;
+};
+// z: the two ring layers and the fraction; zc: the voxel coordinate
+struct SecZ {
+  uint32_t z0, z1;
+  float f, zc;
+};
+
+// Texel-space position u * n - 0.5 of a tile axis of n texels, clamped.
+__device__ __forceinline__ void tile_axis(float u, uint32_t n, SecAxis &a) {
+  a.i0 = floor_frac(clamp_(fmaf(u, (float)n, -0.5f), 0.0f, (float)(n - 1u)), a.f);
+  a.d = a.i0 + 1u < n ? 1u : 0u;
 }
 
-__device__ __forceinline__ float slab_tile(const DevSlab &sl, int L, uint32_t k, float u, float v,
-                                           float w) {
+// REPEAT addressing of the z ring at w = frac(zq): floor(w * wz - 0.5) lies
+// in [-1, wz - 1] and its ring layer is one conditional away.
+__device__ __forceinline__ SecZ ring_axis(float zc, float zq, uint32_t wz) {
+  SecZ z;
+  const float tz = fmaf(zq - floorf(zq), (float)wz, -0.5f);
+  // floor of |tz| < 2^22 by an add that rounds down at 1.5 * 2^23
+  const float r = __fadd_rd(tz, 12582912.0f);
+  z.f = tz - (r - 12582912.0f);
+  const int zi = (int)(__float_as_uint(r) - 0x4B400000u);
+  z.z0 = zi < 0 ? wz - 1u : min((uint32_t)zi, wz - 1u);
+  z.z1 = z.z0 + 1u < wz ? z.z0 + 1u : 0u;
+  z.zc = zc;
+  return z;
+}
+
+// Linear, clamp to edge in x and y (the apron makes tiles seamless), in a
+// tile of rows of tw texels and layers of `plane` texels.
+__device__ __forceinline__ float tile_fetch(const uint8_t *__restrict__ g, uint32_t tw,
+                                            uint32_t plane, const SecAxis &x, const SecAxis &y,
+                                            const SecZ &z) {
+  const uint32_t at = y.i0 * tw + x.i0, dy = y.d ? tw : 0u;
+  const uint8_t *a = g + (size_t)z.z0 * plane + at, *b = g + (size_t)z.z1 * plane + at;
+  const uint8_t *a1 = a + dy, *b1 = b + dy;
+  const float c00 = lerp_raw(raw_u8(a), raw_u8(a + x.d), x.f);
+  const float c10 = lerp_raw(raw_u8(a1), raw_u8(a1 + x.d), x.f);
+  const float c01 = lerp_raw(raw_u8(b), raw_u8(b + x.d), x.f);
+  const float c11 = lerp_raw(raw_u8(b1), raw_u8(b1 + x.d), x.f);
+  return lerp_(lerp_(c00, c10, y.f), lerp_(c01, c11, y.f), z.f) * kInv255;
+}
+
+// a whole float in [0, 2^23) as an integer
+__device__ __forceinline__ uint32_t whole(float x) {
+  return __float_as_uint(x + 8388608.0f) & 0x7fffffu;
+}
+__device__ __forceinline__ float exp2_neg(int k) {  // 2^-k
+  return __uint_as_float((uint32_t)(127 - k) << 23);
+}
+
+// vol_sample of the tiled slab (raycast.slang:423-455): voxel coordinates
+// of p, the ring coordinate, then the overview level whose prefilter
+// (4 << level) matches the footprint, or the base tile under p.  Levels:
+// 0 the base, k + 1 overview k.
+__device__ __forceinline__ int slab_level(const DevSlab &sl, float lod) {
+  const int lev = (int)floorf(lod) - 2;
+  return lev >= 0 ? min(lev, sl.nov - 1) + 1 : 0;
+}
+__device__ __forceinline__ SecAxis slab_axis(const DevSlab &sl, int L, int axis, float p) {
+  const DevSlab::Axis &c = sl.ax[L][axis];
+  const float w = p * sl.nx;
+  // division by the power of two 4 << (L - 1) is exact as a product
+  const float wl = L ? w * exp2_neg(L + 1) : w;
+  SecAxis a;
+  float f;
+  const uint32_t i = floor_frac(r3d_div_by(fmaxf(wl, 0.0f), c.p, c.rp), f);
+  a.q = fminf(__uint_as_float(i | 0x4B000000u) - 8388608.0f, c.gmax);
+  tile_axis(r3d_div_by((wl - a.q * c.p) + 1.0f, c.t, c.rt),
+            (axis ? sl.lev[L].py : sl.lev[L].px) + 2u, a);
+  return a;
+}
+__device__ __forceinline__ SecZ slab_z(const DevSlab &sl, float p) {
+  const float zc = (sl.z0 + 0.5f) + p * sl.nx;
+  return ring_axis(zc, r3d_div_by(zc, (float)sl.wz, sl.rwz), sl.wz);  // frac: the ring wraps
+}
+__device__ __forceinline__ float slab_fetch(const DevSlab &sl, int L, const SecAxis &x,
+                                            const SecAxis &y, const SecZ &z) {
   const DevSlabLevel &lv = sl.lev[L];
-  const uint32_t tw = lv.px + 2u, th = lv.py + 2u, wz = sl.wz;
-  return tex_wrapz(sl.pool + lv.off + (size_t)k * tw * th * wz, tw, th, wz, u, v, w);
+  const uint32_t tw = lv.px + 2u, plane = tw * (lv.py + 2u);
+  const uint32_t k = whole(fmaf(y.q, sl.ax[L][0].gmax + 1.0f, x.q));
+  return tile_fetch(sl.pool + lv.off + (size_t)k * ((size_t)plane * sl.wz), tw, plane, x, y, z);
 }
 
 // sample_clip_level (raycast.slang:360-376): level l's texture at p, its z
 // ring wrapping in level slices
 // (divisions by the powers of two 2^l and 2048 are exact as products)
-__device__ __forceinline__ float clip_level(const DevClip &cl, int l, float3 p) {
-  const float is = 1.0f / (float)(1u << l);
-  const float wx = p.x * cl.nx, wy = p.y * cl.nx;
-  const float zw = (cl.z0 + 0.5f) + p.z * cl.nx;
-  const float u = fmaf(wx - cl.ox[l], is, 1.0f) * (1.0f / 2048.0f);
-  const float v = fmaf(wy - cl.oy[l], is, 1.0f) * (1.0f / 2048.0f);
-  const float zq = (zw * is) / (float)cl.wzl[l];
-  return tex_wrapz(cl.lev[l], 2048u, 2048u, cl.wzl[l], u, v, zq - floorf(zq));
+__device__ __forceinline__ SecAxis clip_axis(const DevClip &cl, int l, int axis, float p) {
+  SecAxis a;
+  const float o = axis ? cl.oy[l] : cl.ox[l];
+  tile_axis(fmaf(p * cl.nx - o, exp2_neg(l), 1.0f) * (1.0f / 2048.0f), 2048u, a);
+  return a;
+}
+__device__ __forceinline__ SecZ clip_z(const DevClip &cl, int l, float p) {
+  const float zw = (cl.z0 + 0.5f) + p * cl.nx;
+  return ring_axis(zw, r3d_div_by(zw * exp2_neg(l), (float)cl.wzl[l], cl.rwzl[l]), cl.wzl[l]);
+}
+__device__ __forceinline__ float clip_fetch(const DevClip &cl, int l, const SecAxis &x,
+                                            const SecAxis &y, const SecZ &z) {
+  return tile_fetch(cl.lev[l], 2048u, 2048u * 2048u, x, y, z);
 }
 
 // pick_clip_level (raycast.slang:380-395): the finest valid level holding
@@ -676,7 +754,7 @@ __device__ __forceinline__ int clip_pick(const DevClip &cl, float3 p, float lod)
     if (li > 5) li = 5 - step;
     if (li < 0) continue;
     if (!(cl.valid & (1u << li))) continue;
-    const float is = 1.0f / (float)(1u << li);  // exact: a power of two
+    const float is = exp2_neg(li);
     const float tx = fmaf(wx - cl.ox[li], is, 1.0f), ty = fmaf(wy - cl.oy[li], is, 1.0f);
     if (tx < 1.0f || tx >= 2047.0f || ty < 1.0f || ty >= 2047.0f) continue;
     return li;
@@ -687,73 +765,77 @@ __device__ __forceinline__ int clip_pick(const DevClip &cl, float3 p, float lod)
 // vs_sample (raycast.slang:331-367): the base cell under p must be the one
 // its tile holds and hold the sample's slice span; then the pyramid level
 // whose prefilter (4 << level) matches the footprint, stepping down past
-// absent levels, or the base tile.  Cells convert through int so that the
-// key of a cell left of the volume is defined.
-__device__ __forceinline__ float vs_sample(const DevVslab &v, float3 p, float lod) {
-  const float P = (float)v.px, T = P + 2.0f;
-  const uint32_t Tu = v.px + 2u;
-  const float wx = v.x0 + p.x * v.nx, wy = v.y0 + p.y * v.nx;
-  const float zc = (v.z0 + 0.5f) + p.z * v.nx;
-  const float zq = zc / (float)v.wz, w = zq - floorf(zq);
-  const float gx0 = (float)v.gx[0], gy0 = (float)v.gy[0];
-  const float cbx = floorf(wx / P), cby = floorf(wy / P);
-  const float pbx = cbx - floorf(cbx / gx0) * gx0, pby = cby - floorf(cby / gy0) * gy0;
-  const uint32_t want = ((uint32_t)(int32_t)cbx & 1023u) |
-                        (((uint32_t)(int32_t)cby & 1023u) << 10) | 0x80000000u;
-  const uint32_t slot = (uint32_t)(pby * gx0 + pbx);
-  const uint4 e = __ldg(reinterpret_cast<const uint4 *>(v.table) + slot);
-  if (e.x != want) return 0.0f;  // not resident
-  if (zc - 0.5f < (float)e.y || zc + 0.5f > (float)e.z) return 0.0f;
+// absent levels, or the base tile.  Levels: 0 the base, l the pyramid's.
+// Cells convert through int so that the key of a cell left of the volume is
+// defined.
+__device__ __forceinline__ int vs_level(const DevVslab &v, float lod) {
   int lev = min((int)floorf(lod) - 2, 3);
   while (lev >= 0 && v.gx[lev + 1] == 0u) lev--;
-  if (lev < 0) {
-    const float lx = (wx - cbx * P) + 1.0f, ly = (wy - cby * P) + 1.0f;
-    return tex_wrapz(v.tiles + (size_t)slot * v.tile_bytes, Tu, Tu, v.wz, lx / T, ly / T, w);
+  return max(lev, -1) + 1;  // fine footprints (lev = -2 or -1): the base
+}
+__device__ __forceinline__ SecAxis vs_axis(const DevVslab &v, int L, int axis, float p) {
+  const float P = (float)v.px, T = P + 2.0f;
+  const float w = (axis ? v.y0 : v.x0) + p * v.nx;
+  const float g0 = (float)(axis ? v.gy[0] : v.gx[0]);
+  const float cb = floorf(r3d_div_by(w, P, v.rp));
+  SecAxis a;
+  a.b = cb - floorf(r3d_div_by(cb, g0, v.rg[0][axis])) * g0;
+  a.key = (uint32_t)(int32_t)cb & 1023u;
+  float c = cb, t = w;
+  a.q = a.b;
+  if (L) {
+    const float g = (float)(axis ? v.gy[L] : v.gx[L]);
+    t = w * exp2_neg(L + 1);
+    c = floorf(r3d_div_by(t, P, v.rp));
+    a.q = c - floorf(r3d_div_by(c, g, v.rg[L][axis])) * g;
   }
-  const int L = lev + 1;
-  const float isc = 1.0f / (float)(4 << lev);  // exact: a power of two
-  const float gxl = (float)v.gx[L], gyl = (float)v.gy[L];
-  const float tx = wx * isc, ty = wy * isc;
-  const float cx = floorf(tx / P), cy = floorf(ty / P);
-  const float qx = cx - floorf(cx / gxl) * gxl, qy = cy - floorf(cy / gyl) * gyl;
-  const float lx = (tx - cx * P) + 1.0f, ly = (ty - cy * P) + 1.0f;
-  const uint32_t k = v.base[L] + (uint32_t)(qy * gxl + qx);
-  return tex_wrapz(v.tiles + (size_t)k * v.tile_bytes, Tu, Tu, v.wz, lx / T, ly / T, w);
+  tile_axis(r3d_div_by((t - c * P) + 1.0f, T, v.rt), v.px + 2u, a);
+  return a;
+}
+__device__ __forceinline__ SecZ vs_z(const DevVslab &v, float p) {
+  const float zc = (v.z0 + 0.5f) + p * v.nx;
+  return ring_axis(zc, r3d_div_by(zc, (float)v.wz, v.rwz), v.wz);
+}
+__device__ __forceinline__ float vs_fetch(const DevVslab &v, int L, const SecAxis &x,
+                                          const SecAxis &y, const SecZ &z) {
+  // (converted saturating: a NaN position, from a NaN camera, stays in range)
+  const uint32_t slot = (uint32_t)(y.b * (float)v.gx[0] + x.b);
+  const uint4 e = __ldg(reinterpret_cast<const uint4 *>(v.table) + slot);
+  if (e.x != (x.key | (y.key << 10) | 0x80000000u)) return 0.0f;  // not resident
+  if (z.zc - 0.5f < (float)e.y || z.zc + 0.5f > (float)e.z) return 0.0f;
+  const uint32_t T = v.px + 2u;
+  const uint32_t k = L ? v.base[L] + (uint32_t)(y.q * (float)v.gx[L] + x.q) : slot;
+  return tile_fetch(v.tiles + (size_t)k * v.tile_bytes, T, T * T, x, y, z);
 }
 
+// The three section paths by their common steps.  L is the level of the
+// sample (clipmap: at least 0).
+template <int PATH>
+__device__ __forceinline__ SecAxis sec_axis(const DevScene &s, int L, int axis, float p) {
+  return PATH == PATH_SLAB   ? slab_axis(s.sl, L, axis, p)
+         : PATH == PATH_CLIP ? clip_axis(s.cl, L, axis, p)
+                             : vs_axis(s.vs, L, axis, p);
+}
+template <int PATH>
+__device__ __forceinline__ SecZ sec_z(const DevScene &s, int L, float p) {
+  return PATH == PATH_SLAB ? slab_z(s.sl, p) : PATH == PATH_CLIP ? clip_z(s.cl, L, p) : vs_z(s.vs, p);
+}
+template <int PATH>
+__device__ __forceinline__ float sec_fetch(const DevScene &s, int L, const SecAxis &x,
+                                           const SecAxis &y, const SecZ &z) {
+  return PATH == PATH_SLAB   ? slab_fetch(s.sl, L, x, y, z)
+         : PATH == PATH_CLIP ? clip_fetch(s.cl, L, x, y, z)
+                             : vs_fetch(s.vs, L, x, y, z);
+}
+template <int PATH>
+__device__ __forceinline__ float sec_sample(const DevScene &s, int L, float3 p) {
+  return sec_fetch<PATH>(s, L, sec_axis<PATH>(s, L, 0, p.x), sec_axis<PATH>(s, L, 1, p.y),
+                         sec_z<PATH>(s, L, p.z));
+}
 // vol_sample in clip mode (raycast.slang:400-403)
-__device__ __forceinline__ float clip_sample(const DevClip &cl, float3 p, float lod) {
+__device__ __forceinline__ float clip_sample(const DevClip &cl, const DevScene &s, float3 p, float lod) {
   const int l = clip_pick(cl, p, lod);
-  return l < 0 ? 0.0f : clip_level(cl, l, p);
-}
-
-// vol_sample of the tiled slab (raycast.slang:423-455): voxel coordinates
-// of p, the ring coordinate, then the overview level whose prefilter
-// (4 << level) matches the footprint, or the base tile under p.
-__device__ __forceinline__ float slab_sample(const DevSlab &sl, float3 p, float lod) {
-  const float wx = p.x * sl.nx, wy = p.y * sl.nx;
-  const float zc = (sl.z0 + 0.5f) + p.z * sl.nx;
-  const float zq = zc / (float)sl.wz;
-  const float w = zq - floorf(zq);  // frac: the ring wraps
-  int lev = (int)floorf(lod) - 2;
-  if (lev >= 0) {
-    lev = min(lev, sl.nov - 1);
-    const float gxl = sl.ov[lev][0], gyl = sl.ov[lev][1], pxl = sl.ov[lev][2], pyl = sl.ov[lev][3];
-    // division by the power of two 4 << lev is exact as a product
-    const float isc = 1.0f / (float)(4 << lev);
-    const float wxl = wx * isc, wyl = wy * isc;
-    const float oix = fminf(floorf(fmaxf(wxl, 0.0f) / pxl), gxl - 1.0f);
-    const float oiy = fminf(floorf(fmaxf(wyl, 0.0f) / pyl), gyl - 1.0f);
-    const float ou = ((wxl - oix * pxl) + 1.0f) / (pxl + 2.0f);
-    const float ov = ((wyl - oiy * pyl) + 1.0f) / (pyl + 2.0f);
-    return slab_tile(sl, lev + 1, (uint32_t)(oiy * gxl + oix), ou, ov, w);
-  }
-  const uint32_t gx = sl.lev[0].gx, gy = sl.lev[0].gy;
-  const uint32_t ix = min((uint32_t)(fmaxf(wx, 0.0f) / sl.px), gx - 1u);
-  const uint32_t iy = min((uint32_t)(fmaxf(wy, 0.0f) / sl.py), gy - 1u);
-  const float u = ((wx - (float)ix * sl.px) + 1.0f) / (sl.px + 2.0f);
-  const float v = ((wy - (float)iy * sl.py) + 1.0f) / (sl.py + 2.0f);
-  return slab_tile(sl, 0, iy * gx + ix, u, v, w);
+  return l < 0 ? 0.0f : sec_sample<PATH_CLIP>(s, l, p);
 }
 
 // Page entry of brick bi of the shard (raycast.slang:813-821); a slot
@@ -1053,16 +1135,12 @@ __device__ __forceinline__ float skip_block(const RayState &st, float3 p, float 
   return fmaxf(fminf(fminf(tex[0], tex[1]), tex[2]), st.t) + bsz * 0.01f;
 }
 
-// A gradient tap: the tiled slab's vol_sample; in clip mode the level the
-// sample picked (or, without one, vol_sample; raycast.slang:942-946,
-// 967-974); else a cube-like texture.
+// The level a section sample was looked up at: its taps read the same one
+// (clipmap: the level the sample picked; raycast.slang:942-946,967-974).
 template <int PATH>
-__device__ __forceinline__ float tap_sample(const DevScene &s, const DevCube &tex, float3 p,
-                                            float lod, int clip_l) {
-  if (PATH == PATH_SLAB) return slab_sample(s.sl, p, lod);
-  if (PATH == PATH_VSLAB) return vs_sample(s.vs, p, lod);
-  if (PATH == PATH_CLIP) return clip_l >= 0 ? clip_level(s.cl, clip_l, p) : clip_sample(s.cl, p, lod);
-  return cube_sample(tex, p, lod);
+__device__ __forceinline__ int sec_level(const DevScene &s, const Pending &q) {
+  return PATH == PATH_SLAB ? slab_level(s.sl, q.lod)
+                           : PATH == PATH_CLIP ? (int)q.slot : vs_level(s.vs, q.lod);
 }
 
 // Colour of a contributing sample: the TF colour, gradient shading (FULL
@@ -1084,7 +1162,6 @@ __device__ __forceinline__ float3 sample_color(const DevScene &s, const ViewCons
   }
   // taps sampled like a cube texture: the cube, or the identity shard atlas
   const DevCube &tex = kShard ? s.sh.atlas : s.cube;
-  constexpr bool kSlab = PATH == PATH_SLAB;
   // non-identity shard: taps at lod_step voxels through the slot
   // (raycast.slang:937-940,972-979)
   const bool slot_taps = kShard && !s.sh.identity;
@@ -1121,28 +1198,29 @@ __device__ __forceinline__ float3 sample_color(const DevScene &s, const ViewCons
         q1 = shard_fetch(s.sh, org, make_float3(u.x - ev, u.y - ev, u.z + ev), q.lod, e2);
         q2 = shard_fetch(s.sh, org, make_float3(u.x - ev, u.y + ev, u.z - ev), q.lod, e2);
         q3 = shard_fetch(s.sh, org, make_float3(u.x + ev, u.y + ev, u.z + ev), q.lod, e2);
-      } else if (kSection) {
-        // one inlined copy of the section lookup, looped over the taps, so
-        // that the kernel stays in the instruction cache
+      } else if (kSection) {  // two values per axis: (+--), (--+), (-+-), (+++)
         const float ee = (vc.voxel * q.lod_step) * ir3;
-        q0 = q1 = q2 = q3 = 0.0f;
-#pragma unroll 1
-        for (int k = 0; k < 4; k++) {  // signs (+--), (--+), (-+-), (+++)
-          const float dx = (k == 0 || k == 3) ? ee : -ee, dy = k >= 2 ? ee : -ee;
-          const float dz = (k & 1) ? ee : -ee;
-          const float t = tap_sample<PATH>(s, tex, make_float3(q.p.x + dx, q.p.y + dy, q.p.z + dz),
-                                           q.lod, (int)q.slot);
-          if (k == 0) q0 = t;
-          else if (k == 1) q1 = t;
-          else if (k == 2) q2 = t;
-          else q3 = t;
+        if (PATH == PATH_CLIP && (int)q.slot < 0) {  // no level at the sample: each tap its own
+          q0 = clip_sample(s.cl, s, make_float3(q.p.x + ee, q.p.y - ee, q.p.z - ee), q.lod);
+          q1 = clip_sample(s.cl, s, make_float3(q.p.x - ee, q.p.y - ee, q.p.z + ee), q.lod);
+          q2 = clip_sample(s.cl, s, make_float3(q.p.x - ee, q.p.y + ee, q.p.z - ee), q.lod);
+          q3 = clip_sample(s.cl, s, make_float3(q.p.x + ee, q.p.y + ee, q.p.z + ee), q.lod);
+        } else {
+          const int L = sec_level<PATH>(s, q);
+          const SecAxis xp = sec_axis<PATH>(s, L, 0, q.p.x + ee), xm = sec_axis<PATH>(s, L, 0, q.p.x - ee);
+          const SecAxis yp = sec_axis<PATH>(s, L, 1, q.p.y + ee), ym = sec_axis<PATH>(s, L, 1, q.p.y - ee);
+          const SecZ zp = sec_z<PATH>(s, L, q.p.z + ee), zm = sec_z<PATH>(s, L, q.p.z - ee);
+          q0 = sec_fetch<PATH>(s, L, xp, ym, zm);
+          q1 = sec_fetch<PATH>(s, L, xm, ym, zp);
+          q2 = sec_fetch<PATH>(s, L, xm, yp, zm);
+          q3 = sec_fetch<PATH>(s, L, xp, yp, zp);
         }
       } else {
         float ee = (vc.voxel * q.lod_step) * ir3;
-        q0 = tap_sample<PATH>(s, tex, make_float3(q.p.x + ee, q.p.y - ee, q.p.z - ee), q.lod, (int)q.slot);
-        q1 = tap_sample<PATH>(s, tex, make_float3(q.p.x - ee, q.p.y - ee, q.p.z + ee), q.lod, (int)q.slot);
-        q2 = tap_sample<PATH>(s, tex, make_float3(q.p.x - ee, q.p.y + ee, q.p.z - ee), q.lod, (int)q.slot);
-        q3 = tap_sample<PATH>(s, tex, make_float3(q.p.x + ee, q.p.y + ee, q.p.z + ee), q.lod, (int)q.slot);
+        q0 = cube_sample(tex, make_float3(q.p.x + ee, q.p.y - ee, q.p.z - ee), q.lod);
+        q1 = cube_sample(tex, make_float3(q.p.x - ee, q.p.y - ee, q.p.z + ee), q.lod);
+        q2 = cube_sample(tex, make_float3(q.p.x - ee, q.p.y + ee, q.p.z - ee), q.lod);
+        q3 = cube_sample(tex, make_float3(q.p.x + ee, q.p.y + ee, q.p.z + ee), q.lod);
       }
       g0 = (((q0 - q1) - q2) + q3) * renorm;
       g1 = (((-q0 - q1) + q2) + q3) * renorm;
@@ -1188,36 +1266,61 @@ __device__ __forceinline__ float3 sample_color(const DevScene &s, const ViewCons
              shard_fetch(s.sh, org, make_float3(u.x, u.y - ev, u.z), q.lod, e2);
         g2 = shard_fetch(s.sh, org, make_float3(u.x, u.y, u.z + ev), q.lod, e2) -
              shard_fetch(s.sh, org, make_float3(u.x, u.y, u.z - ev), q.lod, e2);
-      } else if (kSection) {  // looped taps, as above
+      } else if (kSection) {  // a tap moves one axis of the sample's lookup
         const float e = vc.voxel * q.lod_step;
-        float plus = 0.0f;
-        g0 = g1 = g2 = 0.0f;
+        if (PATH == PATH_CLIP && (int)q.slot < 0) {  // as above
+          g0 = clip_sample(s.cl, s, make_float3(q.p.x + e, q.p.y, q.p.z), q.lod) -
+               clip_sample(s.cl, s, make_float3(q.p.x - e, q.p.y, q.p.z), q.lod);
+          g1 = clip_sample(s.cl, s, make_float3(q.p.x, q.p.y + e, q.p.z), q.lod) -
+               clip_sample(s.cl, s, make_float3(q.p.x, q.p.y - e, q.p.z), q.lod);
+          g2 = clip_sample(s.cl, s, make_float3(q.p.x, q.p.y, q.p.z + e), q.lod) -
+               clip_sample(s.cl, s, make_float3(q.p.x, q.p.y, q.p.z - e), q.lod);
+        } else {
+          const int L = sec_level<PATH>(s, q);
+          const SecAxis x = sec_axis<PATH>(s, L, 0, q.p.x), y = sec_axis<PATH>(s, L, 1, q.p.y);
+          const SecZ z = sec_z<PATH>(s, L, q.p.z);
+          if constexpr (PATH == PATH_VSLAB) {
+            // its axes are long (two cells each): looped over one copy of the
+            // lookup, so that the kernel stays in the instruction cache (six
+            // copies: 1.23 ms a frame, `no_instruction` the top stall; looped
+            // 1.15.  The slab and the clipmap run 7 % faster with six)
+            float plus = 0.0f;
+            g0 = g1 = g2 = 0.0f;
 #pragma unroll 1
-        for (int k = 0; k < 6; k++) {  // +x, -x, +y, -y, +z, -z
-          const int ax = k >> 1;
-          const float d = (k & 1) ? -e : e;
-          const float t = tap_sample<PATH>(
-              s, tex,
-              make_float3(ax == 0 ? q.p.x + d : q.p.x, ax == 1 ? q.p.y + d : q.p.y,
-                          ax == 2 ? q.p.z + d : q.p.z),
-              q.lod, (int)q.slot);
-          if (!(k & 1)) {
-            plus = t;
+            for (int k = 0; k < 6; k++) {  // +x, -x, +y, -y, +z, -z
+              const float d = (k & 1) ? -e : e;
+              SecAxis tx = x, ty = y;
+              SecZ tz = z;
+              if (k < 4) {
+                const SecAxis t = sec_axis<PATH>(s, L, k >> 1, (k < 2 ? q.p.x : q.p.y) + d);
+                if (k < 2) tx = t;
+                else ty = t;
+              } else {
+                tz = sec_z<PATH>(s, L, q.p.z + d);
+              }
+              const float t = sec_fetch<PATH>(s, L, tx, ty, tz);
+              if (!(k & 1)) plus = t;
+              else if (k == 1) g0 = plus - t;
+              else if (k == 3) g1 = plus - t;
+              else g2 = plus - t;
+            }
           } else {
-            const float g = plus - t;
-            if (ax == 0) g0 = g;
-            else if (ax == 1) g1 = g;
-            else g2 = g;
+            g0 = sec_fetch<PATH>(s, L, sec_axis<PATH>(s, L, 0, q.p.x + e), y, z) -
+                 sec_fetch<PATH>(s, L, sec_axis<PATH>(s, L, 0, q.p.x - e), y, z);
+            g1 = sec_fetch<PATH>(s, L, x, sec_axis<PATH>(s, L, 1, q.p.y + e), z) -
+                 sec_fetch<PATH>(s, L, x, sec_axis<PATH>(s, L, 1, q.p.y - e), z);
+            g2 = sec_fetch<PATH>(s, L, x, y, sec_z<PATH>(s, L, q.p.z + e)) -
+                 sec_fetch<PATH>(s, L, x, y, sec_z<PATH>(s, L, q.p.z - e));
           }
         }
       } else {
         float e = vc.voxel * q.lod_step;
-        g0 = tap_sample<PATH>(s, tex, make_float3(q.p.x + e, q.p.y, q.p.z), q.lod, (int)q.slot) -
-             tap_sample<PATH>(s, tex, make_float3(q.p.x - e, q.p.y, q.p.z), q.lod, (int)q.slot);
-        g1 = tap_sample<PATH>(s, tex, make_float3(q.p.x, q.p.y + e, q.p.z), q.lod, (int)q.slot) -
-             tap_sample<PATH>(s, tex, make_float3(q.p.x, q.p.y - e, q.p.z), q.lod, (int)q.slot);
-        g2 = tap_sample<PATH>(s, tex, make_float3(q.p.x, q.p.y, q.p.z + e), q.lod, (int)q.slot) -
-             tap_sample<PATH>(s, tex, make_float3(q.p.x, q.p.y, q.p.z - e), q.lod, (int)q.slot);
+        g0 = cube_sample(tex, make_float3(q.p.x + e, q.p.y, q.p.z), q.lod) -
+             cube_sample(tex, make_float3(q.p.x - e, q.p.y, q.p.z), q.lod);
+        g1 = cube_sample(tex, make_float3(q.p.x, q.p.y + e, q.p.z), q.lod) -
+             cube_sample(tex, make_float3(q.p.x, q.p.y - e, q.p.z), q.lod);
+        g2 = cube_sample(tex, make_float3(q.p.x, q.p.y, q.p.z + e), q.lod) -
+             cube_sample(tex, make_float3(q.p.x, q.p.y, q.p.z - e), q.lod);
       }
     }
     float3 gv = make_float3(g0, g1, g2);
@@ -1350,10 +1453,13 @@ __device__ __forceinline__ int ray_step(const DevScene &s, const ViewConst &vc, 
   float lod = 0.0f;
   bool lod_known = true;
   if (vc.lod_on) {
-    if (kLod && t >= st.lod_tlo && t < st.lod_thi)
+    if (kLod && t >= st.lod_tlo && t < st.lod_thi) {
       lod_known = false;  // level and lod_step known (lod_range)
-    else
-      lod = clamp_(r3d_log2f(lod_y(vc, t)) + vc.lod_bias, 0.0f, vc.max_lod);
+    } else {
+      // a footprint under a voxel is clamped to y = 1, whose logarithm is 0
+      const float y = lod_y(vc, t);
+      lod = clamp_((!kLod && y == 1.0f ? 0.0f : r3d_log2f(y)) + vc.lod_bias, 0.0f, vc.max_lod);
+    }
   }
   float lod_step =
       !lod_known || st.span_dom ? st.span_step
@@ -1453,13 +1559,13 @@ __device__ __forceinline__ int ray_step(const DevScene &s, const ViewConst &vc, 
                : 0.0f;
     }
   } else if (kSlab) {
-    v = slab_sample(s.sl, p, lod);
+    v = sec_sample<PATH_SLAB>(s, slab_level(s.sl, lod), p);
   } else if (kVslab) {
-    v = vs_sample(s.vs, p, lod);
+    v = sec_sample<PATH_VSLAB>(s, vs_level(s.vs, lod), p);
   } else if (kClip) {  // the level is picked once; taps reuse it (raycast.slang:785-787)
     const int cl = clip_pick(s.cl, p, lod);
     b.slot = (uint32_t)cl;
-    v = cl < 0 ? 0.0f : clip_level(s.cl, cl, p);
+    v = cl < 0 ? 0.0f : sec_sample<PATH_CLIP>(s, cl, p);
   } else {
     v = cube_sample(s.cube, p, lod);
   }

@@ -160,17 +160,18 @@ int r3d_cuda_slab_build(r3d_cuda_ctx *c, const r3d_volume_desc *d, const uint8_t
   sl.ny = (float)ny;
   sl.px = (float)base.px;
   sl.py = (float)base.py;
-  // the overview branch's per-level constants, in the shader's float
-  // expressions (raycast.slang:430-446)
+  sl.rwz = 1.0f / (float)wz;
+  // the axis constants of the base, then of the overview levels in the
+  // shader's float expressions (raycast.slang:430-446)
   sl.nov = (int)(r3d_log2f((float)ovs) + 0.5f) - 1;
-  for (int k = 0; k < sl.nov && k < kSlabLevels; k++) {
-    const float sc = (float)(4 << k);
-    const float vnx = ceilf(sl.nx / sc), vny = ceilf(sl.ny / sc);
-    const float gxl = ceilf(vnx / 2046.0f), gyl = ceilf(vny / 2046.0f);
-    sl.ov[k][0] = gxl;
-    sl.ov[k][1] = gyl;
-    sl.ov[k][2] = ceilf(vnx / gxl);
-    sl.ov[k][3] = ceilf(vny / gyl);
+  for (int L = 0; L <= sl.nov && L < kSlabLevels; L++) {
+    const float n[2] = {sl.nx, sl.ny}, bp[2] = {sl.px, sl.py};
+    const float bg[2] = {(float)base.gx, (float)base.gy}, sc = L ? (float)(4 << (L - 1)) : 1.0f;
+    for (int a = 0; a < 2; a++) {
+      const float vn = ceilf(n[a] / sc), g = L ? ceilf(vn / 2046.0f) : bg[a];
+      const float p = L ? ceilf(vn / g) : bp[a];
+      sl.ax[L][a] = {p, 1.0f / p, p + 2.0f, 1.0f / (p + 2.0f), g - 1.0f};
+    }
   }
   size_t off = 0, planes = 0;
   for (uint32_t lev = 0; lev < sl.nlev; lev++) {

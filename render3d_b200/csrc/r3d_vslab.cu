@@ -215,7 +215,12 @@ int r3d_cuda_vslab_begin(r3d_cuda_ctx *c, const r3d_volume_desc *d, const uint8_
     dv.gx[l] = v.gx[l];
     dv.gy[l] = v.gy[l];
     dv.base[l] = v.base[l];
+    dv.rg[l][0] = v.gx[l] ? 1.0f / (float)v.gx[l] : 0.0f;
+    dv.rg[l][1] = v.gy[l] ? 1.0f / (float)v.gy[l] : 0.0f;
   }
+  dv.rp = 1.0f / (float)v.px;
+  dv.rt = 1.0f / ((float)v.px + 2.0f);
+  dv.rwz = 1.0f / (float)v.wz;
   dv.nx = (float)v.W;
   c->vs = dv;
   c->have_vslab = true;
