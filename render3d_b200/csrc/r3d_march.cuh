@@ -1766,6 +1766,28 @@ struct ShadeQueue {
   uint32_t own[32];  // per ray: its entries of the batch
 };
 
+// Folds the colours and weights that stand in entries [head, head + n) of a
+// (64 entries, n <= 32; lane l < n brought the entry's ray) into the rays'
+// sums, oldest first; own: 32 words of the warp.
+__device__ __forceinline__ void shade_fold(float4 *a, uint32_t *own, uint32_t head, uint32_t n,
+                                           uint32_t ray, float &acc_r, float &acc_g, float &acc_b) {
+  constexpr uint32_t kAll = 0xffffffffu;
+  const uint32_t lane = threadIdx.x & 31u;
+  const bool mine = lane < n;
+  own[lane] = 0u;
+  const uint32_t peers = __match_any_sync(kAll, mine ? ray : 32u + lane);
+  __syncwarp();
+  if (mine) own[ray] = peers;
+  __syncwarp();
+  for (uint32_t m = own[lane]; m; m &= m - 1u) {
+    const float4 c = a[(head + (uint32_t)__ffs((int)m) - 1u) & 63u];
+    acc_r = fmaf(c.w, c.x, acc_r);
+    acc_g = fmaf(c.w, c.y, acc_g);
+    acc_b = fmaf(c.w, c.z, acc_b);
+  }
+  __syncwarp();
+}
+
 // Shades the n <= 32 oldest entries (from head), all lanes together.
 template <int PATH, int MODE, bool FAST>
 __device__ __forceinline__ void shade_batch(const DevScene &s, const ViewConst &vc,
@@ -1778,8 +1800,6 @@ __device__ __forceinline__ void shade_batch(const DevScene &s, const ViewConst &
   const uint32_t tag = __float_as_uint(B.w), ray = tag & 31u;
   const float3 dir = make_float3(__shfl_sync(kAll, st.dir.x, ray), __shfl_sync(kAll, st.dir.y, ray),
                                  __shfl_sync(kAll, st.dir.z, ray));
-  q.own[lane] = 0u;
-  const uint32_t peers = __match_any_sync(kAll, mine ? ray : 32u + lane);
   if (mine) {
     Pending p;
     p.p = p.bl = make_float3(A.x, A.y, A.z);
@@ -1791,16 +1811,7 @@ __device__ __forceinline__ void shade_batch(const DevScene &s, const ViewConst &
     const float3 c = sample_color<PATH, MODE, FAST>(s, vc, dir, p);
     q.a[e] = make_float4(c.x, c.y, c.z, B.z);
   }
-  __syncwarp();
-  if (mine) q.own[ray] = peers;
-  __syncwarp();
-  for (uint32_t m = q.own[lane]; m; m &= m - 1u) {
-    const float4 c = q.a[(head + (uint32_t)__ffs((int)m) - 1u) & 63u];
-    st.acc_r = fmaf(c.w, c.x, st.acc_r);
-    st.acc_g = fmaf(c.w, c.y, st.acc_g);
-    st.acc_b = fmaf(c.w, c.z, st.acc_b);
-  }
-  __syncwarp();
+  shade_fold(q.a, q.own, head, n, ray, st.acc_r, st.acc_g, st.acc_b);
 }
 
 // Whether a kernel's FULL views shade through the queue when the schedule

@@ -177,6 +177,7 @@ struct DevSurfView {
   uint32_t gw, gh;
   const uint8_t *mask;  // supervision mask, or null
   uint32_t mw, mh;
+  float ix, iy, iz;  // 1 / W, 1 / H, 1 / L as the view's parameters give them
 };
 
 // Clamp-to-edge trilinear of the (R, G) volume at normalized uvw.
@@ -250,187 +251,318 @@ __device__ __forceinline__ float2 surf_layer(const uint16_t *__restrict__ vol, s
 
 enum SurfKind { kSurfFull = 0, kSurfFlat = 1, kSurfMip = 2, kSurfStretch = 3 };
 
-// The surf branch of the raycast (raycast.slang:515-638) for one pixel.  The
-// ray runs along the layers at fixed (u, v), and a trilinear sample lerps x,
-// then y, then z: so the (x, y) lerps of a layer are shared by every sample
-// between it and its neighbours.  The column's value at the two layers of
-// the sample is kept and shifted as the ray passes a layer, and so are the
-// values of the four columns that the in-plane gradient taps read, from the
-// first contributing sample on; the two taps along the layers read the
-// column itself.  The same operations in the same order, with four texels
-// read per column and layer instead of eight per sample and tap.
-template <int KIND, bool OVL>
-__device__ __forceinline__ float3 surf_pixel(const r3d_frame_params &pc, const DevSurfView &v,
-                                             const float4 *tf, float alpha_cutoff, float tf_zero_t,
-                                             uint32_t px, uint32_t py) {
-  const float3 bg = make_float3(0.02f, 0.02f, 0.03f);
+// One pixel of the surf branch of the raycast (raycast.slang:515-638): where
+// it lies on the segment, and its ray along the layers.
+struct SurfRay {
+  float fu, fv;  // segment coordinates
+  float tx, ty;  // window texels
+  float t, hi, dt, center, lo;
+};
+
+// False: background.
+__device__ __forceinline__ bool surf_begin(const r3d_frame_params &pc, uint32_t px, uint32_t py,
+                                           SurfRay &r) {
   const float ux = ((float)px + 0.5f) / (float)pc.viewport[0];
   const float uy = ((float)py + 0.5f) / (float)pc.viewport[1];
   const float nx = ux * 2.0f - 1.0f, ny = 1.0f - uy * 2.0f;
-  const float fu = fmaf(ny, pc.cam_up[0], fmaf(nx, pc.cam_right[0], pc.cam_origin[0]));
-  const float fv = fmaf(ny, pc.cam_up[1], fmaf(nx, pc.cam_right[1], pc.cam_origin[1]));
-  const float tx = (fu - pc.slab_x0) / pc.slab_px, ty = (fv - pc.slab_y0) / pc.slab_px;
-  if (tx < 0.0f || ty < 0.0f || tx >= pc.slab_nx || ty >= pc.slab_ny) return bg;
+  r.fu = fmaf(ny, pc.cam_up[0], fmaf(nx, pc.cam_right[0], pc.cam_origin[0]));
+  r.fv = fmaf(ny, pc.cam_up[1], fmaf(nx, pc.cam_right[1], pc.cam_origin[1]));
+  r.tx = (r.fu - pc.slab_x0) / pc.slab_px;
+  r.ty = (r.fv - pc.slab_y0) / pc.slab_px;
+  if (r.tx < 0.0f || r.ty < 0.0f || r.tx >= pc.slab_nx || r.ty >= pc.slab_ny) return false;
   const float L = (float)pc.slab_wz;
-  const float center = (pc.slab_z0 - pc.max_mip) + (float)(pc.slab_grid & 0xffffu);
+  r.center = (pc.slab_z0 - pc.max_mip) + (float)(pc.slab_grid & 0xffffu);
   const float halfd = 0.5f * fmaxf((float)pc.slab_depth, 1.0f);
-  const float lo = clamp_(center - halfd, 0.0f, L), hi = clamp_(center + halfd, 0.0f, L);
-  if (lo >= hi) return bg;
-  const float ix = 1.0f / pc.slab_nx, iy = 1.0f / pc.slab_ny, iz = 1.0f / L;
-  if (KIND == kSurfStretch) {  // flattening-distortion heatmap (:540-570)
-    const float gx = fu * pc.vol_tx, gy = fv * pc.vol_ty;
-    const int gix = (int)clamp_(gx, 1.0f, (float)v.gw - 2.0f);
-    const int giy = (int)clamp_(gy, 1.0f, (float)v.gh - 2.0f);
-    const float4 cu0 = v.coords[(size_t)giy * v.gw + gix - 1], cu1 = v.coords[(size_t)giy * v.gw + gix + 1];
-    const float4 cv0 = v.coords[(size_t)(giy - 1) * v.gw + gix], cv1 = v.coords[(size_t)(giy + 1) * v.gw + gix];
-    if (fminf(fminf(cu0.w, cu1.w), fminf(cv0.w, cv1.w)) < 0.5f) return bg;
-    const float3 du = make_float3(cu1.x - cu0.x, cu1.y - cu0.y, cu1.z - cu0.z);
-    const float3 dv = make_float3(cv1.x - cv0.x, cv1.y - cv0.y, cv1.z - cv0.z);
-    const float su = sqrtf(dot3(du, du)) * 0.5f * pc.vol_tx;
-    const float sv = sqrtf(dot3(dv, dv)) * 0.5f * pc.vol_ty;
-    const float x = clamp_(r3d_log2f(fmaxf(0.5f * (su + sv), 1e-4f)) / 0.35f, -1.0f, 1.0f);
-    const float m = r3d_powf(fabsf(x), 0.6f);
-    const float3 tint = x < 0.0f ? make_float3(0.0f, 0.35f, 1.0f) : make_float3(1.0f, 0.15f, 0.0f);
-    const float ct = surf_tex(v, tx * ix, ty * iy, clamp_(center, lo, hi) * iz).x;
-    const float k = fmaf(0.5f, ct, 0.5f);
-    return make_float3(lerp_(0.95f, tint.x, m) * k, lerp_(0.95f, tint.y, m) * k,
-                       lerp_(0.95f, tint.z, m) * k);
-  }
-  constexpr bool composite = KIND != kSurfMip;
-  const float dt = fmaxf(pc.step_voxels, 0.25f);  // layers per step
-  float t = fmaf(hash12(px, py, pc.frame_index), dt, lo);
-  float mip_max = 0.0f, ink_max = 0.0f;
-  float acc_r = 0.0f, acc_g = 0.0f, acc_b = 0.0f, acc_a = 0.0f;
-  const float3 oc = flat_overlay_color(pc.overlay_flags);
-  const float opac_k = pc.density * pc.step_voxels;
-  const float u = tx * ix, w = ty * iy;
-  const uint16_t *vol = reinterpret_cast<const uint16_t *>(v.vol);
-  const size_t plane = (size_t)v.W * v.H;
-  const SurfAxis cx = surf_axis(u, v.W), cy = surf_axis(w, v.H);
-  // the column at layers have and have + 1 (clamped; 0xffffffff: none yet),
-  // and its texels at the layer after those, loaded one layer ahead of use
-  SurfTexels ahead = {0u, 0u, 0u, 0u};
-  uint32_t have = 0xffffffffu, have4 = 0xffffffffu;
-  float2 e0 = make_float2(0.0f, 0.0f), e1 = e0;
-  float q0[4] = {0.0f, 0.0f, 0.0f, 0.0f}, q1[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // u+, u-, w+, w-
-  SurfAxis xp = cx, xm = cx, yp = cy, ym = cy;
-  for (uint32_t k = 0; k < 512u && t < hi; k++, t += dt) {
-    const float z = t * iz;
-    const SurfAxis cz = surf_axis(z, v.L);
-    if (cz.i0 != have) {
-      const bool next = cz.i0 == have + 1u && have != 0xffffffffu;
-      e0 = next ? e1 : surf_layer<OVL>(vol, plane, v.W, cz.i0, cx, cy);
-      if (!next) ahead = surf_texels(vol, plane, v.W, cz.i0 + cz.d, cx, cy);
-      e1 = surf_lerp<OVL>(ahead, cx, cy);  // (the last layer: e0 again)
-      have = cz.i0;
-      ahead = surf_texels(vol, plane, v.W, min(have + 2u, v.L - 1u), cx, cy);
-    }
-    const float val = lerp_(e0.x, e1.x, cz.f) * kInv255;
-    const float ink = OVL ? lerp_(e0.y, e1.y, cz.f) * kInv255 : 0.0f;
-    if (OVL && ink > ink_max) ink_max = ink;
-    if (val < pc.threshold) continue;
-    if (!composite) {
-      if (val > mip_max) mip_max = val;
-      continue;
-    }
-    const float tt = clamp_(fmaf(val, 256.0f, -0.5f), 0.0f, 255.0f);
-    if (tt < tf_zero_t) continue;  // both TF texels have alpha 0: the opacity is 1 - 1^k = 0
-    const float4 sm = tf_sample(tf, tt);
-    const float a = 1.0f - r3d_powf(1.0f - sm.w, opac_k);
-    if (a <= 0.003f) continue;
-    float cr = sm.x, cg = sm.y, cb = sm.z;
-    if (KIND == kSurfFull) {  // 1-texel taps in flattened space
-      if (have4 != cz.i0) {
-        if (have4 == 0xffffffffu) {
-          xp = surf_axis(u + ix, v.W);
-          xm = surf_axis(u - ix, v.W);
-          yp = surf_axis(w + iy, v.H);
-          ym = surf_axis(w - iy, v.H);
-        }
-        const bool next = cz.i0 == have4 + 1u && have4 != 0xffffffffu;
-        if (next) {
-#pragma unroll
-          for (int i = 0; i < 4; i++) q0[i] = q1[i];
-        } else {
-          q0[0] = surf_layer<false>(vol, plane, v.W, cz.i0, xp, cy).x;
-          q0[1] = surf_layer<false>(vol, plane, v.W, cz.i0, xm, cy).x;
-          q0[2] = surf_layer<false>(vol, plane, v.W, cz.i0, cx, yp).x;
-          q0[3] = surf_layer<false>(vol, plane, v.W, cz.i0, cx, ym).x;
-        }
-        if (cz.d) {
-          q1[0] = surf_layer<false>(vol, plane, v.W, cz.i0 + 1u, xp, cy).x;
-          q1[1] = surf_layer<false>(vol, plane, v.W, cz.i0 + 1u, xm, cy).x;
-          q1[2] = surf_layer<false>(vol, plane, v.W, cz.i0 + 1u, cx, yp).x;
-          q1[3] = surf_layer<false>(vol, plane, v.W, cz.i0 + 1u, cx, ym).x;
-        } else {
-#pragma unroll
-          for (int i = 0; i < 4; i++) q1[i] = q0[i];
-        }
-        have4 = cz.i0;
-      }
-      const float g0 = lerp_(q0[0], q1[0], cz.f) * kInv255 - lerp_(q0[1], q1[1], cz.f) * kInv255;
-      const float g1 = lerp_(q0[2], q1[2], cz.f) * kInv255 - lerp_(q0[3], q1[3], cz.f) * kInv255;
-      // the taps along the layers: mostly one layer off the sample's pair
-      const SurfAxis zp = surf_axis(z + iz, v.L), zm = surf_axis(z - iz, v.L);
-      const auto at = [&](uint32_t l) {
-        return l == cz.i0 ? e0.x : l == cz.i0 + cz.d ? e1.x
-                                 : surf_layer<false>(vol, plane, v.W, l, cx, cy).x;
-      };
-      const float p0 = at(zp.i0), p1 = at(zp.i0 + zp.d), m0 = at(zm.i0), m1 = at(zm.i0 + zm.d);
-      const float g2 = lerp_(p0, p1, zp.f) * kInv255 - lerp_(m0, m1, zm.f) * kInv255;
-      const float gm = sqrtf(fmaf(g2, g2, fmaf(g1, g1, g0 * g0)));
-      if (gm > 1e-4f) {
-        const float diff = fmaf(0.7f, fabsf(g2 / gm), 0.3f);  // headlight along the layers
-        const float lit = fmaf(0.75f, diff, 0.25f);
-        const float lm = lerp_(1.0f, lit, sat_(gm * 6.0f));
-        cr *= lm, cg *= lm, cb *= lm;
-      }
-    }
-    if (OVL) {
-      const float kk = sat_(ink * pc.overlay_gain);
-      cr = lerp_(cr, oc.x, kk), cg = lerp_(cg, oc.y, kk), cb = lerp_(cb, oc.z, kk);
-    }
-    const float wgt = (1.0f - acc_a) * a;
-    acc_r = fmaf(wgt, cr, acc_r);
-    acc_g = fmaf(wgt, cg, acc_g);
-    acc_b = fmaf(wgt, cb, acc_b);
-    acc_a = acc_a + wgt;
-    if (acc_a >= alpha_cutoff) break;
-  }
-  float3 col;
-  if (composite) {
-    const float tr = 1.0f - acc_a;
-    col = make_float3(fmaf(tr, bg.x, acc_r), fmaf(tr, bg.y, acc_g), fmaf(tr, bg.z, acc_b));
-  } else {
-    const float m = mip_max * pc.density;
-    col = make_float3(m, m, m);
-    if (OVL) {
-      const float kk = sat_(ink_max * pc.overlay_gain);
-      col = make_float3(lerp_(col.x, oc.x, kk), lerp_(col.y, oc.y, kk), lerp_(col.z, oc.z, kk));
-    }
-  }
-  if ((pc.overlay_flags & 32u) && v.mask) {  // supervision mask, nearest (:619-635)
-    const float gx = fu * pc.vol_tx, gy = fv * pc.vol_ty;
-    const float upx = (float)v.mw / fmaxf((float)v.gw - 1.0f, 1.0f);
-    const float upy = (float)v.mh / fmaxf((float)v.gh - 1.0f, 1.0f);
-    const float mxf = gx * upx, myf = gy * upy;
-    // int(g * up) truncates toward zero, so (-1, 0) lands on texel 0
-    if (mxf > -1.0f && myf > -1.0f && mxf < (float)v.mw && myf < (float)v.mh) {
-      const int mx = (int)mxf, my = (int)myf;
-      const uint32_t mc = v.mask[(size_t)my * v.mw + mx];
-      if (mc == 1u)
-        col = make_float3(lerp_(col.x, 0.25f, 0.45f), lerp_(col.y, 0.45f, 0.45f), lerp_(col.z, 1.0f, 0.45f));
-      else if (mc >= 2u)
-        col = make_float3(lerp_(col.x, 1.0f, 0.55f), lerp_(col.y, 0.55f, 0.55f), lerp_(col.z, 0.10f, 0.55f));
-    }
+  r.lo = clamp_(r.center - halfd, 0.0f, L);
+  r.hi = clamp_(r.center + halfd, 0.0f, L);
+  if (r.lo >= r.hi) return false;
+  r.dt = fmaxf(pc.step_voxels, 0.25f);  // layers per step
+  r.t = fmaf(hash12(px, py, pc.frame_index), r.dt, r.lo);
+  return true;
+}
+
+// The flattening-distortion heatmap (:540-570).
+__device__ __forceinline__ float3 surf_stretch(const r3d_frame_params &pc, const DevSurfView &v,
+                                               const SurfRay &r) {
+  const float ix = v.ix, iy = v.iy, iz = v.iz;
+  const float gx = r.fu * pc.vol_tx, gy = r.fv * pc.vol_ty;
+  const int gix = (int)clamp_(gx, 1.0f, (float)v.gw - 2.0f);
+  const int giy = (int)clamp_(gy, 1.0f, (float)v.gh - 2.0f);
+  const float4 cu0 = v.coords[(size_t)giy * v.gw + gix - 1], cu1 = v.coords[(size_t)giy * v.gw + gix + 1];
+  const float4 cv0 = v.coords[(size_t)(giy - 1) * v.gw + gix], cv1 = v.coords[(size_t)(giy + 1) * v.gw + gix];
+  if (fminf(fminf(cu0.w, cu1.w), fminf(cv0.w, cv1.w)) < 0.5f) return make_float3(0.02f, 0.02f, 0.03f);
+  const float3 du = make_float3(cu1.x - cu0.x, cu1.y - cu0.y, cu1.z - cu0.z);
+  const float3 dv = make_float3(cv1.x - cv0.x, cv1.y - cv0.y, cv1.z - cv0.z);
+  const float su = sqrtf(dot3(du, du)) * 0.5f * pc.vol_tx;
+  const float sv = sqrtf(dot3(dv, dv)) * 0.5f * pc.vol_ty;
+  const float x = clamp_(r3d_log2f(fmaxf(0.5f * (su + sv), 1e-4f)) / 0.35f, -1.0f, 1.0f);
+  const float m = r3d_powf(fabsf(x), 0.6f);
+  const float3 tint = x < 0.0f ? make_float3(0.0f, 0.35f, 1.0f) : make_float3(1.0f, 0.15f, 0.0f);
+  const float ct = surf_tex(v, r.tx * ix, r.ty * iy, clamp_(r.center, r.lo, r.hi) * iz).x;
+  const float k = fmaf(0.5f, ct, 0.5f);
+  return make_float3(lerp_(0.95f, tint.x, m) * k, lerp_(0.95f, tint.y, m) * k,
+                     lerp_(0.95f, tint.z, m) * k);
+}
+
+// The supervision mask over a pixel's colour, nearest (:619-635).
+__device__ __forceinline__ float3 surf_mask(const r3d_frame_params &pc, const DevSurfView &v,
+                                            const SurfRay &r, float3 col) {
+  if (!(pc.overlay_flags & 32u) || !v.mask) return col;
+  const float gx = r.fu * pc.vol_tx, gy = r.fv * pc.vol_ty;
+  const float upx = (float)v.mw / fmaxf((float)v.gw - 1.0f, 1.0f);
+  const float upy = (float)v.mh / fmaxf((float)v.gh - 1.0f, 1.0f);
+  const float mxf = gx * upx, myf = gy * upy;
+  // int(g * up) truncates toward zero, so (-1, 0) lands on texel 0
+  if (mxf > -1.0f && myf > -1.0f && mxf < (float)v.mw && myf < (float)v.mh) {
+    const int mx = (int)mxf, my = (int)myf;
+    const uint32_t mc = v.mask[(size_t)my * v.mw + mx];
+    if (mc == 1u)
+      col = make_float3(lerp_(col.x, 0.25f, 0.45f), lerp_(col.y, 0.45f, 0.45f), lerp_(col.z, 1.0f, 0.45f));
+    else if (mc >= 2u)
+      col = make_float3(lerp_(col.x, 1.0f, 0.55f), lerp_(col.y, 0.55f, 0.55f), lerp_(col.z, 0.10f, 0.55f));
   }
   return col;
 }
 
+// The column of a ray, layer by layer.  The ray runs along the layers at
+// fixed (u, v), and a trilinear sample lerps x, then y, then z: so the (x, y)
+// lerps of a layer are shared by every sample between it and its neighbours.
+// The column's values at the two layers of the sample are kept and shifted
+// as the ray passes a layer, and its texels at the layer after those are
+// loaded one layer ahead of use.
+template <bool G>
+struct SurfColumn {
+  SurfAxis x, y;
+  uint32_t have = 0xffffffffu;  // the lower layer held
+  float2 e0, e1;
+  SurfTexels ahead;
+  __device__ __forceinline__ void move(const uint16_t *__restrict__ vol, size_t plane, uint32_t W,
+                                       uint32_t L, const SurfAxis &z) {
+    if (z.i0 == have) return;
+    const bool next = z.i0 == have + 1u && have != 0xffffffffu;
+    e0 = next ? e1 : surf_layer<G>(vol, plane, W, z.i0, x, y);
+    if (!next) ahead = surf_texels(vol, plane, W, z.i0 + z.d, x, y);
+    e1 = surf_lerp<G>(ahead, x, y);  // (the last layer: e0 again)
+    have = z.i0;
+    ahead = surf_texels(vol, plane, W, min(have + 2u, L - 1u), x, y);
+  }
+};
+
+// The shading queue of a warp (see ShadeQueue): per entry the sample's z, TF
+// coordinate, weight and ink, then its colour and weight.
+struct SurfQueue {
+  float4 a[64];
+  uint8_t ray[64];
+  uint32_t own[32];
+};
+
+// R of the texels at p[x], as 2^23 + byte
+__device__ __forceinline__ float surf_raw(const uint16_t *__restrict__ p, int x) {
+  return qraw(__ldg(p + x), 0);
+}
+
+// The cross of a sample at one layer, away from the volume's edges: the
+// values of its column and of the columns one texel along x and y, from the
+// twelve texels that they read between them (20 column by column).
+struct SurfCross {
+  float c, xp, xm, yp, ym;
+};
+struct SurfFrac {  // fractions of the sample and of its taps
+  float x, xp, xm, y, yp, ym;
+};
+__device__ __forceinline__ SurfCross surf_cross(const uint16_t *__restrict__ p, int W,
+                                                const SurfFrac &f) {
+  const uint16_t *r1 = p + W, *rm = p - W, *r2 = r1 + W;
+  const float a0 = surf_raw(p, -1), b0 = surf_raw(p, 0), c0 = surf_raw(p, 1), d0 = surf_raw(p, 2);
+  const float a1 = surf_raw(r1, -1), b1 = surf_raw(r1, 0), c1 = surf_raw(r1, 1), d1 = surf_raw(r1, 2);
+  const float bm = surf_raw(rm, 0), cm = surf_raw(rm, 1), b2 = surf_raw(r2, 0), c2 = surf_raw(r2, 1);
+  const float x0 = lerp_raw(b0, c0, f.x), x1 = lerp_raw(b1, c1, f.x);
+  SurfCross s;
+  s.c = lerp_(x0, x1, f.y);
+  s.xp = lerp_(lerp_raw(c0, d0, f.xp), lerp_raw(c1, d1, f.xp), f.y);
+  s.xm = lerp_(lerp_raw(a0, b0, f.xm), lerp_raw(a1, b1, f.xm), f.y);
+  s.yp = lerp_(x1, lerp_raw(b2, c2, f.x), f.yp);
+  s.ym = lerp_(lerp_raw(bm, cm, f.x), x0, f.ym);
+  return s;
+}
+
+// Colour of the contributing sample at (u, w, z): TF colour, shading by
+// 1-texel taps in flattened space, ink tint.  A tap is a trilinear lookup;
+// the four in-plane ones share the sample's layers and fraction along them,
+// the two along the layers its column.
+template <bool OVL>
+__device__ __forceinline__ float3 surf_shade(const r3d_frame_params &pc, const DevSurfView &v,
+                                             const float4 *tf, float u, float w, float z, float tt,
+                                             float ink) {
+  const float ix = v.ix, iy = v.iy, iz = v.iz;
+  const uint16_t *vol = reinterpret_cast<const uint16_t *>(v.vol);
+  const size_t plane = (size_t)v.W * v.H;
+  const SurfAxis x = surf_axis(u, v.W), y = surf_axis(w, v.H), c = surf_axis(z, v.L);
+  const SurfAxis zp = surf_axis(z + iz, v.L), zm = surf_axis(z - iz, v.L);
+  const auto at = [&](uint32_t l, const SurfAxis &ax, const SurfAxis &ay) {
+    return surf_layer<false>(vol, plane, v.W, l, ax, ay).x;
+  };
+  const auto tap = [&](const SurfAxis &ax, const SurfAxis &ay, const SurfAxis &az) {
+    return lerp_(at(az.i0, ax, ay), at(az.i0 + az.d, ax, ay), az.f) * kInv255;
+  };
+  const SurfAxis xp = surf_axis(u + ix, v.W), xm = surf_axis(u - ix, v.W);
+  const SurfAxis yp = surf_axis(w + iy, v.H), ym = surf_axis(w - iy, v.H);
+  float g0, g1, g2;
+  // every tap exactly one texel off, none clamped at an edge (a tap's own
+  // rounding can put it in the sample's texel, or two off)
+  if (x.i0 - 1u < v.W - 3u && y.i0 - 1u < v.H - 3u && c.i0 - 1u < v.L - 3u && v.W > 3u &&
+      v.H > 3u && v.L > 3u && xp.i0 == x.i0 + 1u && xm.i0 + 1u == x.i0 && yp.i0 == y.i0 + 1u &&
+      ym.i0 + 1u == y.i0 && zp.i0 == c.i0 + 1u && zm.i0 + 1u == c.i0) {
+    const uint16_t *p = vol + c.i0 * plane + (size_t)y.i0 * v.W + x.i0;
+    const SurfFrac f = {x.f, xp.f, xm.f, y.f, yp.f, ym.f};
+    const SurfCross s0 = surf_cross(p, (int)v.W, f), s1 = surf_cross(p + plane, (int)v.W, f);
+    const auto column = [&](const uint16_t *q) {
+      const uint16_t *q1 = q + v.W;
+      return lerp_(lerp_raw(surf_raw(q, 0), surf_raw(q, 1), f.x),
+                   lerp_raw(surf_raw(q1, 0), surf_raw(q1, 1), f.x), f.y);
+    };
+    g0 = lerp_(s0.xp, s1.xp, c.f) * kInv255 - lerp_(s0.xm, s1.xm, c.f) * kInv255;
+    g1 = lerp_(s0.yp, s1.yp, c.f) * kInv255 - lerp_(s0.ym, s1.ym, c.f) * kInv255;
+    g2 = lerp_(s1.c, column(p + 2u * plane), zp.f) * kInv255 -
+         lerp_(column(p - plane), s0.c, zm.f) * kInv255;
+  } else {
+    g0 = tap(xp, y, c) - tap(xm, y, c);
+    g1 = tap(x, yp, c) - tap(x, ym, c);
+    g2 = tap(x, y, zp) - tap(x, y, zm);
+  }
+  const float4 sm = tf_sample(tf, tt);
+  float cr = sm.x, cg = sm.y, cb = sm.z;
+  const float gm = sqrtf(fmaf(g2, g2, fmaf(g1, g1, g0 * g0)));
+  if (gm > 1e-4f) {
+    const float diff = fmaf(0.7f, fabsf(g2 / gm), 0.3f);  // headlight along the layers
+    const float lit = fmaf(0.75f, diff, 0.25f);
+    const float lm = lerp_(1.0f, lit, sat_(gm * 6.0f));
+    cr *= lm, cg *= lm, cb *= lm;
+  }
+  if (OVL) {
+    const float3 oc = flat_overlay_color(pc.overlay_flags);
+    const float kk = sat_(ink * pc.overlay_gain);
+    cr = lerp_(cr, oc.x, kk), cg = lerp_(cg, oc.y, kk), cb = lerp_(cb, oc.z, kk);
+  }
+  return make_float3(cr, cg, cb);
+}
+
+// A warp's 32 pixels (`inside` says whether the lane has one).
+template <int KIND, bool OVL>
+__device__ __forceinline__ float3 surf_pixel(const r3d_frame_params &pc, const DevSurfView &v,
+                                             const float4 *tf, float alpha_cutoff, float tf_zero_t,
+                                             uint32_t px, uint32_t py, bool inside, SurfQueue &sq) {
+  constexpr uint32_t kAll = 0xffffffffu;
+  const float3 bg = make_float3(0.02f, 0.02f, 0.03f);
+  SurfRay r;
+  const bool hit = inside && surf_begin(pc, px, py, r);
+  if (KIND == kSurfStretch) return hit ? surf_stretch(pc, v, r) : bg;
+  constexpr bool composite = KIND != kSurfMip, queued = KIND == kSurfFull;
+  const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+  const float iz = v.iz;
+  const float u = hit ? r.tx * v.ix : 0.0f, w = hit ? r.ty * v.iy : 0.0f;
+  const float3 oc = flat_overlay_color(pc.overlay_flags);
+  const float opac_k = pc.density * pc.step_voxels;
+  const uint16_t *vol = reinterpret_cast<const uint16_t *>(v.vol);
+  const size_t plane = (size_t)v.W * v.H;
+  SurfColumn<OVL> col;
+  col.x = surf_axis(u, v.W);
+  col.y = surf_axis(w, v.H);
+  float mip_max = 0.0f, ink_max = 0.0f;
+  float acc_r = 0.0f, acc_g = 0.0f, acc_b = 0.0f, acc_a = 0.0f;
+  float t = hit ? r.t : 0.0f;
+  const float hi = hit ? r.hi : 0.0f;
+  uint32_t head = 0, n = 0;  // the queue's waiting entries: [head, head + n), mod 64
+  const auto shade = [&](uint32_t k) {
+    const uint32_t e = (head + lane) & 63u;
+    const float4 A = sq.a[e];
+    const uint32_t ray = sq.ray[e] & 31u;
+    const float ru = __shfl_sync(kAll, u, ray), rw = __shfl_sync(kAll, w, ray);
+    if (lane < k) {
+      const float3 c = surf_shade<OVL>(pc, v, tf, ru, rw, A.x, A.y, A.w);
+      sq.a[e] = make_float4(c.x, c.y, c.z, A.z);
+    }
+    shade_fold(sq.a, sq.own, head, k, ray, acc_r, acc_g, acc_b);
+    head += k;
+    n -= k;
+  };
+  bool active = hit;
+  uint32_t k = 0;
+  while (queued ? __any_sync(kAll, active) : active) {
+    bool push = false;
+    float z = 0.0f, tt = 0.0f, wgt = 0.0f, ink = 0.0f;
+    if (active && !(k < 512u && t < hi)) active = false;
+    if (active) {
+      z = t * iz;
+      const SurfAxis cz = surf_axis(z, v.L);
+      col.move(vol, plane, v.W, v.L, cz);
+      const float val = lerp_(col.e0.x, col.e1.x, cz.f) * kInv255;
+      ink = OVL ? lerp_(col.e0.y, col.e1.y, cz.f) * kInv255 : 0.0f;
+      if (OVL && ink > ink_max) ink_max = ink;
+      if (!(val < pc.threshold)) {
+        if (!composite && val > mip_max) mip_max = val;
+        tt = clamp_(fmaf(val, 256.0f, -0.5f), 0.0f, 255.0f);
+        // below tf_zero_t both TF texels have alpha 0: the opacity is 1 - 1^k = 0
+        if (composite && !(tt < tf_zero_t)) {
+          const float4 sm = tf_sample(tf, tt);
+          const float a = 1.0f - r3d_powf(1.0f - sm.w, opac_k);
+          if (a > 0.003f) {
+            wgt = (1.0f - acc_a) * a;
+            if (!queued) {
+              float cr = sm.x, cg = sm.y, cb = sm.z;
+              if (OVL) {
+                const float kk = sat_(ink * pc.overlay_gain);
+                cr = lerp_(cr, oc.x, kk), cg = lerp_(cg, oc.y, kk), cb = lerp_(cb, oc.z, kk);
+              }
+              acc_r = fmaf(wgt, cr, acc_r);
+              acc_g = fmaf(wgt, cg, acc_g);
+              acc_b = fmaf(wgt, cb, acc_b);
+            }
+            push = true;
+            acc_a = acc_a + wgt;
+            if (acc_a >= alpha_cutoff) active = false;
+          }
+        }
+      }
+      k++;
+      t += r.dt;
+    }
+    if (queued) {
+      const uint32_t add = __ballot_sync(kAll, push);
+      if (add) {
+        if (push) {
+          const uint32_t e = (head + n + (uint32_t)__popc(add & below)) & 63u;
+          sq.a[e] = make_float4(z, tt, wgt, ink);
+          sq.ray[e] = (uint8_t)lane;
+        }
+        n += (uint32_t)__popc(add);
+        __syncwarp();
+        if (n >= 32u) shade(32u);
+      }
+    }
+  }
+  if (queued && n) shade(n);  // at most 31 are left
+  if (!hit) return bg;
+  float3 c;
+  if (composite) {
+    const float tr = 1.0f - acc_a;
+    c = make_float3(fmaf(tr, bg.x, acc_r), fmaf(tr, bg.y, acc_g), fmaf(tr, bg.z, acc_b));
+  } else {
+    const float m = mip_max * pc.density;
+    c = make_float3(m, m, m);
+    if (OVL) {
+      const float kk = sat_(ink_max * pc.overlay_gain);
+      c = make_float3(lerp_(c.x, oc.x, kk), lerp_(c.y, oc.y, kk), lerp_(c.z, oc.z, kk));
+    }
+  }
+  return surf_mask(pc, v, r, c);
+}
+
 // One thread per pixel, 8x4 Morton warp tiles.  Bound by issue: at 1600x900
 // over a 1536^2 x 80 window, FULL, 1.45 ms with eight texels per sample and
-// tap, 0.88 ms with the columns' layers kept, 0.83 ms with the next layer's
-// texels loaded ahead.
+// tap, 0.88 ms with the column's layers kept, 0.83 ms with the next layer's
+// texels loaded ahead, 0.68 ms with the taps through the warp's queue and
+// their texels shared (0.83 with the queue alone; FLAT, without taps: 0.33).
 template <int KIND, bool OVL>
 __global__ void __launch_bounds__(128) k_surf_raycast(const __grid_constant__ r3d_frame_params pc,
                                                       const __grid_constant__ DevSurfView v,
@@ -440,6 +572,7 @@ __global__ void __launch_bounds__(128) k_surf_raycast(const __grid_constant__ r3
                                                       uint32_t *__restrict__ steps_out,
                                                       uint32_t *__restrict__ mip_out) {
   __shared__ float4 tf[256];
+  __shared__ SurfQueue sq[KIND == kSurfFull ? 4 : 1];
   for (uint32_t i = threadIdx.x; i < 256u; i += blockDim.x) {
     const uchar4 u = lut[i];
     tf[i] = make_float4((float)u.x, (float)u.y, (float)u.z, (float)u.w);
@@ -452,8 +585,10 @@ __global__ void __launch_bounds__(128) k_surf_raycast(const __grid_constant__ r3
   const uint32_t ty = blockIdx.y * 8u + (warp >> 1) * 4u + (((lane >> 1) & 1u) | ((lane >> 2) & 2u));
   const uint32_t px = half ? tx * 2u : tx, py = half ? ty * 2u : ty;
   const uint32_t vw = pc.viewport[0], vh = pc.viewport[1];
-  if (px >= vw || py >= vh) return;
-  const float3 c = surf_pixel<KIND, OVL>(pc, v, tf, alpha_cutoff, tf_zero_t, px, py);
+  const bool inside = px < vw && py < vh;
+  const float3 c = surf_pixel<KIND, OVL>(pc, v, tf, alpha_cutoff, tf_zero_t, px, py, inside,
+                                         sq[KIND == kSurfFull ? warp : 0u]);
+  if (!inside) return;
   const uchar4 col = make_uchar4(unorm8(c.x), unorm8(c.y), unorm8(c.z), 255);
   const uint32_t ox = pc.view_org & 0xffffu, oy = pc.view_org >> 16;
   for (uint32_t k = 0; k < (half ? 4u : 1u); k++) {
@@ -475,6 +610,7 @@ cudaError_t launch_surf(const r3d_cuda_ctx *c, const r3d_frame_params &pc, uint8
   v.gw = c->surf_gw, v.gh = c->surf_gh;
   v.mask = c->surf_mask;
   v.mw = c->surf_mw, v.mh = c->surf_mh;
+  v.ix = 1.0f / pc.slab_nx, v.iy = 1.0f / pc.slab_ny, v.iz = 1.0f / (float)pc.slab_wz;
   const bool half = (pc.view_flags & R3D_VIEW_HALF) != 0u;
   const uint32_t gw = half ? (pc.viewport[0] + 1u) / 2u : pc.viewport[0];
   const uint32_t gh = half ? (pc.viewport[1] + 1u) / 2u : pc.viewport[1];
