@@ -30,6 +30,36 @@ __device__ __forceinline__ uint2 load8(const uint8_t *__restrict__ row, uint32_t
   return make_uint2(load4<false>(row, x, n), load4<false>(row, x + 4u, n));
 }
 
+// A warp writes dst[0, n): byte i is row[x0 + i], row[0] left of the row, and
+// past its nx bytes row[nx - 1] (CLAMP) or 0.  Words of dst are stored whole
+// and read as two aligned words of the row; only its unaligned ends and the
+// words that leave the row go byte by byte.
+template <bool CLAMP>
+__device__ __forceinline__ uint32_t row_byte(const uint8_t *__restrict__ row, int64_t x, uint32_t nx) {
+  if (x >= (int64_t)nx) return CLAMP ? row[nx - 1u] : 0u;
+  return row[x < 0 ? 0 : x];
+}
+template <bool CLAMP>
+__device__ __forceinline__ void warp_row(uint8_t *__restrict__ dst, uint32_t n,
+                                         const uint8_t *__restrict__ row, int64_t x0, uint32_t nx) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t head = min((uint32_t)(-(uintptr_t)dst & 3u), n), words = (n - head) / 4u;
+  const uint32_t tail = head + words * 4u;
+  if (lane < head) dst[lane] = (uint8_t)row_byte<CLAMP>(row, x0 + lane, nx);
+  if (tail + lane < n) dst[tail + lane] = (uint8_t)row_byte<CLAMP>(row, x0 + tail + lane, nx);
+  for (uint32_t k = lane; k < words; k += 32u) {
+    const int64_t x = x0 + head + 4u * k;
+    uint32_t v = 0;
+    if (x >= 0 && x + 4 <= (int64_t)nx) {
+      v = load4<false>(row, (uint32_t)x, nx);
+    } else {
+#pragma unroll
+      for (int b = 0; b < 4; b++) v |= row_byte<CLAMP>(row, x + b, nx) << (8 * b);
+    }
+    *reinterpret_cast<uint32_t *>(dst + head + 4u * k) = v;
+  }
+}
+
 // the largest of the four bytes of w
 __device__ __forceinline__ uint32_t max_byte(uint32_t w) {
   w = __vmaxu4(w, w >> 16);

@@ -10,6 +10,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "r3d_build.cuh"
 #include "r3d_internal.h"
 
 namespace r3d {
@@ -30,42 +31,58 @@ __global__ void k_clip_down2(const uint8_t *__restrict__ src, uint32_t sx, uint3
   }
 }
 
-// One ring layer of level l holding level slice ls (vkclip.c:101-185):
-// level 0 is the volume, level 1 the 2^3 box (truncating) of the volume with
-// coordinates clamped at full resolution, levels 2.. the pyramid clamped at
-// their own extent; texel (tx, ty) is level voxel (vx0 + tx, vy0 + ty);
-// slices outside the volume are zero.
-__global__ void k_clip_fill(const uint8_t *__restrict__ vol, uint32_t nx, uint32_t ny, uint32_t nz,
-                            const uint8_t *__restrict__ pyr, uint32_t lx, uint32_t ly,
-                            uint32_t lz, uint32_t l, int64_t vx0, int64_t vy0, int64_t ls,
-                            uint8_t *__restrict__ layer) {
-  const size_t n = (size_t)kClipTex * kClipTex;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const int64_t tx = (int64_t)(i % kClipTex), ty = (int64_t)(i / kClipTex);
-    uint32_t v = 0;
-    if (l == 0u) {
-      if (ls >= 0 && ls < (int64_t)nz) {
-        const int64_t x = min(max(vx0 + tx, (int64_t)0), (int64_t)nx - 1);
-        const int64_t y = min(max(vy0 + ty, (int64_t)0), (int64_t)ny - 1);
-        v = vol[((size_t)ls * ny + (size_t)y) * nx + (size_t)x];
+// Ring layers, one job each: a layer of level l holding level slice ls
+// (vkclip.c:101-185): level 0 is the volume, level 1 the 2^3 box (truncating)
+// of the volume with coordinates clamped at full resolution, levels 2.. the
+// pyramid clamped at their own extent; texel (tx, ty) is level voxel (vx0 +
+// tx, vy0 + ty); slices outside the volume are zero.  One warp per row of a
+// layer, words of four texels, all layers of a frame in one launch (a launch
+// per 4 MiB layer with a byte a thread took 16 us each).
+struct ClipJob {
+  const uint8_t *src;  // the level's volume: its bytes and extent
+  uint32_t nx, ny, nz, l;
+  int64_t vx0, vy0, ls;
+  uint8_t *layer;
+};
+constexpr uint32_t kClipJobs = 48u;
+struct ClipJobs {
+  ClipJob j[kClipJobs];
+};
+__global__ void __launch_bounds__(256) k_clip_fill(const __grid_constant__ ClipJobs jobs) {
+  const ClipJob &c = jobs.j[blockIdx.y];
+  const uint32_t lane = threadIdx.x & 31u;
+  for (uint32_t ty = blockIdx.x * 8u + (threadIdx.x >> 5); ty < kClipTex; ty += gridDim.x * 8u) {
+    uint8_t *dst = c.layer + (size_t)ty * kClipTex;
+    if (c.l == 1u) {  // 8 source bytes of four rows to four texels
+      for (uint32_t k = lane; k < kClipTex / 4u; k += 32u) {
+        const int64_t x = 2 * (c.vx0 + 4u * k);
+        uint32_t s0 = 0, s1 = 0;  // sums of texels 0, 1 and 2, 3
+        for (int r = 0; r < 4; r++) {
+          const int64_t z = 2 * c.ls + (r >> 1);
+          if (z < 0 || z >= (int64_t)c.nz) continue;
+          const int64_t y = min(max(2 * (c.vy0 + ty) + (r & 1), (int64_t)0), (int64_t)c.ny - 1);
+          const uint8_t *row = c.src + ((size_t)z * c.ny + (size_t)y) * c.nx;
+          uint2 w = make_uint2(0u, 0u);
+          if (x >= 0 && x + 8 <= (int64_t)c.nx) {
+            w = load8<false>(row, (uint32_t)x, c.nx);
+          } else {
+            for (int b = 0; b < 4; b++) {
+              w.x |= row_byte<true>(row, x + b, c.nx) << (8 * b);
+              w.y |= row_byte<true>(row, x + 4 + b, c.nx) << (8 * b);
+            }
+          }
+          s0 += (w.x & 0x00FF00FFu) + ((w.x >> 8) & 0x00FF00FFu);
+          s1 += (w.y & 0x00FF00FFu) + ((w.y >> 8) & 0x00FF00FFu);
+        }
+        reinterpret_cast<uint32_t *>(dst)[k] =
+            __byte_perm((s0 >> 3) & 0x00FF00FFu, (s1 >> 3) & 0x00FF00FFu, 0x6420);
       }
-    } else if (l == 1u) {
-      uint32_t sum = 0;
-      for (int k = 0; k < 8; k++) {
-        const int64_t z = 2 * ls + (k >> 2);
-        if (z < 0 || z >= (int64_t)nz) continue;
-        const int64_t x = min(max(2 * (vx0 + tx) + (k & 1), (int64_t)0), (int64_t)nx - 1);
-        const int64_t y = min(max(2 * (vy0 + ty) + ((k >> 1) & 1), (int64_t)0), (int64_t)ny - 1);
-        sum += vol[((size_t)z * ny + (size_t)y) * nx + (size_t)x];
-      }
-      v = sum / 8u;
-    } else if (ls >= 0 && ls < (int64_t)lz && lx && ly) {
-      const int64_t x = min(max(vx0 + tx, (int64_t)0), (int64_t)lx - 1);
-      const int64_t y = min(max(vy0 + ty, (int64_t)0), (int64_t)ly - 1);
-      v = pyr[((size_t)ls * ly + (size_t)y) * lx + (size_t)x];
+    } else if (c.ls >= 0 && c.ls < (int64_t)c.nz && c.nx && c.ny) {
+      const int64_t y = min(max(c.vy0 + (int64_t)ty, (int64_t)0), (int64_t)c.ny - 1);
+      warp_row<true>(dst, kClipTex, c.src + ((size_t)c.ls * c.ny + (size_t)y) * c.nx, c.vx0, c.nx);
+    } else {
+      for (uint32_t k = lane; k < kClipTex / 4u; k += 32u) reinterpret_cast<uint32_t *>(dst)[k] = 0u;
     }
-    layer[i] = (uint8_t)v;
   }
 }
 
@@ -172,6 +189,12 @@ int r3d_cuda_clip_frame(r3d_cuda_ctx *c, double fx, double fy, uint64_t z0, r3d_
   cudaSetDevice(c->device);
   const int64_t nx = c->clip_dims[0], ny = c->clip_dims[1];
   const int64_t ifx = (int64_t)fx, ify = (int64_t)fy;
+  ClipJobs jobs;
+  uint32_t nj = 0;
+  const auto launch = [&] {
+    if (nj) k_clip_fill<<<dim3(nj < 4u ? 256u : 64u, nj), 256, 0, c->stream>>>(jobs);
+    nj = 0;
+  };
   for (int l = 0; l < kClipLevels; l++) {
     const int64_t s = (int64_t)1 << l, cov = (int64_t)kClipPayload * s;
     int64_t &ox = c->clip_org[l][0], &oy = c->clip_org[l][1];
@@ -206,15 +229,17 @@ int r3d_cuda_clip_frame(r3d_cuda_ctx *c, double fx, double fy, uint64_t z0, r3d_
       const int64_t ls = ls0 + k;
       const uint32_t layer = (uint32_t)(ls % wzl);
       if (c->clip_layer[l][layer] == ls) continue;
-      k_clip_fill<<<4096, 256, 0, c->stream>>>(
-          c->clip_src, c->clip_dims[0], c->clip_dims[1], c->clip_dims[2], pyr, q[0], q[1], q[2],
-          (uint32_t)l, ox / s - 1, oy / s - 1, ls,
-          const_cast<uint8_t *>(c->cl.lev[l]) + (size_t)layer * kClipTex * kClipTex);
+      const bool vol = l < 2;
+      const uint32_t *e = vol ? c->clip_dims : q;
+      jobs.j[nj++] = {vol ? c->clip_src : pyr, e[0], e[1], e[2], (uint32_t)l, ox / s - 1, oy / s - 1, ls,
+                      const_cast<uint8_t *>(c->cl.lev[l]) + (size_t)layer * kClipTex * kClipTex};
+      if (nj == kClipJobs) launch();
       c->clip_layer[l][layer] = ls;
     }
     c->cl.ox[l] = (float)ox;
     c->cl.oy[l] = (float)oy;
   }
+  launch();
   R3D_CUDA_TRY(c, cudaGetLastError());
   c->cl.valid = (1u << kClipLevels) - 1u;
   c->cl.z0 = (float)z0;

@@ -97,6 +97,8 @@ struct r3d_cuda_ctx {
   std::vector<r3d_vslab_job> vs_jobs;
   r3d_vslab_layout vsl{};
   size_t vs_strip_off[r3d::kVsLevels] = {};
+  size_t vs_strip_bytes = 0;  // one job's strips
+  uint32_t vs_batch = 1;      // jobs whose strips fit the scratch
   bool have_vslab = false;
   r3d::DevVslab vs{};
 

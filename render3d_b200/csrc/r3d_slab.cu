@@ -9,6 +9,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "r3d_build.cuh"
 #include "r3d_internal.h"
 
 namespace r3d {
@@ -54,25 +55,28 @@ __global__ void k_slab_down(const uint8_t *__restrict__ src, uint32_t sx, uint32
 // Tile slices of one level for a run of slices: texel (tx, ty) of tile
 // (i, j) in ring layer (s % wz) is plane[s][row(j, ty)][col(i, tx)] with
 // the apron rows and columns clamped to the plane (slab.h:82-95,
-// vkbackend.c:2148-2164).  Grid: (.., slices).
-__global__ void k_slab_tiles(const uint8_t *__restrict__ plane, size_t plane_stride,
+// vkbackend.c:2148-2164).  One warp per tile row, words of four texels: a
+// slice of 4096^2 took 100 us a byte a thread and takes 20.  Grid: (..,
+// slices).
+__global__ void __launch_bounds__(256) k_slab_tiles(const uint8_t *__restrict__ plane, size_t plane_stride,
                              uint32_t nx, uint32_t ny, uint32_t gx, uint32_t gy, uint32_t px,
                              uint32_t py, uint32_t wz, uint32_t s0, uint8_t *__restrict__ tiles) {
   const uint32_t s = s0 + blockIdx.y, layer = s % wz;
   const uint8_t *p = plane + (size_t)blockIdx.y * plane_stride;
   const uint32_t tw = px + 2u, th = py + 2u;
   const size_t tile_bytes = (size_t)tw * th * wz;
-  const size_t total = (size_t)gx * gy * tw * th;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const uint32_t tx = (uint32_t)(i % tw), ty = (uint32_t)((i / tw) % th);
-    const uint32_t k = (uint32_t)(i / ((size_t)tw * th));
-    const uint32_t ti = k % gx, tj = k / gx;
-    const int64_t cx = min(max((int64_t)ti * px - 1 + tx, (int64_t)0), (int64_t)nx - 1);
+  const uint32_t rows = gx * gy * th;
+  for (uint32_t r = blockIdx.x * 8u + (threadIdx.x >> 5); r < rows; r += gridDim.x * 8u) {
+    const uint32_t ty = r % th, k = r / th, ti = k % gx, tj = k / gx;
     const int64_t cy = min(max((int64_t)tj * py - 1 + ty, (int64_t)0), (int64_t)ny - 1);
-    tiles[(size_t)k * tile_bytes + (size_t)layer * tw * th + (size_t)ty * tw + tx] =
-        p[(size_t)cy * nx + (size_t)cx];
+    warp_row<true>(tiles + (size_t)k * tile_bytes + (size_t)layer * tw * th + (size_t)ty * tw, tw,
+                   p + (size_t)cy * nx, (int64_t)ti * px - 1, nx);
   }
+}
+
+// blocks of a warp per row
+static unsigned slab_rows(const DevSlabLevel &l) {
+  return std::min((l.gx * l.gy * (l.py + 2u) + 7u) / 8u, 148u * 16u);
 }
 
 static unsigned slab_grid1(size_t n) {
@@ -90,8 +94,7 @@ static int slab_fill(r3d_cuda_ctx *c, uint32_t s0, uint32_t s1) {
     const uint32_t n = std::min(16u, s1 - a);
     const uint8_t *src = c->slab_src + (size_t)a * plane;
     const DevSlabLevel &b = sl.lev[0];
-    k_slab_tiles<<<dim3(slab_grid1((size_t)b.gx * b.gy * (b.px + 2u) * (b.py + 2u)), n), 256, 0,
-                   st>>>(src, plane, nx, ny, b.gx, b.gy, b.px, b.py, sl.wz, a,
+    k_slab_tiles<<<dim3(slab_rows(b), n), 256, 0, st>>>(src, plane, nx, ny, b.gx, b.gy, b.px, b.py, sl.wz, a,
                          c->slab_buf + b.off);
     const uint8_t *prev = src;
     uint32_t pnx = nx, pny = ny;
@@ -103,8 +106,7 @@ static int slab_fill(r3d_cuda_ctx *c, uint32_t s0, uint32_t s1) {
       k_slab_down<<<dim3(slab_grid1((size_t)onx * ony), n), 256, 0, st>>>(
           prev, pnx, pny, pstride, dst, onx, ony, (size_t)onx * ony, f);
       const DevSlabLevel &L = sl.lev[lev];
-      k_slab_tiles<<<dim3(slab_grid1((size_t)L.gx * L.gy * (L.px + 2u) * (L.py + 2u)), n), 256,
-                     0, st>>>(dst, (size_t)onx * ony, onx, ony, L.gx, L.gy, L.px, L.py, sl.wz, a,
+      k_slab_tiles<<<dim3(slab_rows(L), n), 256, 0, st>>>(dst, (size_t)onx * ony, onx, ony, L.gx, L.gy, L.px, L.py, sl.wz, a,
                               c->slab_buf + L.off);
       prev = dst;
       pnx = onx;
