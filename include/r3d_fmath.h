@@ -170,4 +170,15 @@ R3D_FM_HD float r3d_div_by(float a, float b, float rb) {
   return fmaf(fmaf(-b, q, a), rb, q);
 }
 
+/* a / b, correctly rounded, for any b with rb = 1 / b (rounded), b, 1 / b and
+ * the quotient normal numbers or a = 0: as above with a second correction.
+ * The first leaves a quotient within an ulp of a / b, whose residual is then
+ * exact, and one more from such a quotient rounds correctly (Markstein's
+ * theorem, as above). */
+R3D_FM_HD float r3d_div_rcp(float a, float b, float rb) {
+  float q = a * rb;
+  q = fmaf(fmaf(-b, q, a), rb, q);
+  return fmaf(fmaf(-b, q, a), rb, q);
+}
+
 #endif /* R3D_FMATH_H */

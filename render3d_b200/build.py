@@ -48,7 +48,7 @@ CU_SOURCES = ["r3d_ctx.cu", "r3d_build.cu", "r3d_fwd.cu", "r3d_persist.cu", "r3d
 # sources compiled once more per sampling path (-DR3D_FWD_PATH=p), so the
 # paths' raycast kernels compile in parallel
 PER_PATH = {"r3d_fwd.cu", "r3d_persist.cu"}
-N_PATHS = 6
+N_PATHS = 8
 C_SOURCES = ["r3d_render.c", "r3d_host.c"]
 CLI_SOURCES = ["r3d_headless.c"]
 

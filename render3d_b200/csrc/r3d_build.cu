@@ -216,4 +216,146 @@ cudaError_t launch_slot_tables(const uint8_t *pool, const uint32_t *slot, uint32
   return cudaGetLastError();
 }
 
+// A warp per output row of the kernels below: words of four bytes a lane,
+// loaded at whatever alignment the row has.
+static unsigned row_blocks(uint64_t rows) {
+  const uint64_t b = (rows + 7u) / 8u;
+  return (unsigned)(b < 148u * 32u ? (b ? b : 1u) : 148u * 32u);
+}
+
+// Next mip: clamped coordinates matter only where the source has one texel
+// (elsewhere 2 d <= s).  The mips of a 1024^3 cube took 0.77 ms a byte a
+// thread; rows that start on 8 bytes are loaded in whole words (VEC), which
+// took a 1024^3 shard build from 2.81 to 2.36 ms.
+template <bool VEC>
+__global__ void __launch_bounds__(256) k_mip(const uint8_t *__restrict__ src, uint32_t sx,
+                                             uint32_t sy, uint32_t sz, uint8_t *__restrict__ dst,
+                                             uint32_t dx, uint32_t dy, uint32_t dz) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint64_t rows = (uint64_t)dy * dz;
+  for (uint64_t r = blockIdx.x * 8ull + (threadIdx.x >> 5); r < rows; r += gridDim.x * 8ull) {
+    const uint32_t y = (uint32_t)(r % dy), z = (uint32_t)(r / dy);
+    for (uint32_t x = lane * 4u; x < dx; x += 128u) {
+      uint32_t s0 = 0x00040004u, s1 = 0x00040004u;
+#pragma unroll
+      for (uint32_t k = 0; k < 4u; k++) {
+        const uint32_t yy = min(2u * y + (k & 1u), sy - 1u), zz = min(2u * z + (k >> 1), sz - 1u);
+        uint2 w = load8<VEC>(src + ((size_t)zz * sy + yy) * sx, 2u * x, sx);
+        if (sx == 1u) w.x |= w.x << 8;
+        s0 += (w.x & 0x00FF00FFu) + ((w.x >> 8) & 0x00FF00FFu);
+        s1 += (w.y & 0x00FF00FFu) + ((w.y >> 8) & 0x00FF00FFu);
+      }
+      const uint32_t v = __byte_perm((s0 >> 3) & 0x00FF00FFu, (s1 >> 3) & 0x00FF00FFu, 0x6420);
+      uint8_t *o = dst + r * dx + x;
+      if (!(dx & 3u)) {
+        *reinterpret_cast<uint32_t *>(o) = v;
+      } else {
+        for (uint32_t k = 0; k < 4u && x + k < dx; k++) o[k] = (uint8_t)(v >> (8u * k));
+      }
+    }
+  }
+}
+
+cudaError_t launch_mip(const uint8_t *src, uint32_t sx, uint32_t sy, uint32_t sz, uint8_t *dst,
+                       uint32_t dx, uint32_t dy, uint32_t dz, cudaStream_t st) {
+  const unsigned grid = row_blocks((uint64_t)dy * dz);
+  if (sx % 8u == 0u && ((uintptr_t)src & 7u) == 0u)
+    k_mip<true><<<grid, 256, 0, st>>>(src, sx, sy, sz, dst, dx, dy, dz);
+  else
+    k_mip<false><<<grid, 256, 0, st>>>(src, sx, sy, sz, dst, dx, dy, dz);
+  return cudaGetLastError();
+}
+
+// 8^3 block maxima (src/vk/vkbackend.c:794-824), a lane per block: eight
+// bytes of each of its 64 rows.
+template <bool VEC>
+__global__ void __launch_bounds__(256) k_occ_raw(const uint8_t *__restrict__ vox, uint32_t nx,
+                                                 uint32_t ny, uint32_t nz,
+                                                 uint8_t *__restrict__ raw, uint32_t ox,
+                                                 uint32_t oy, uint32_t oz) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint64_t rows = (uint64_t)oy * oz;
+  for (uint64_t r = blockIdx.x * 8ull + (threadIdx.x >> 5); r < rows; r += gridDim.x * 8ull) {
+    const uint32_t y0 = (uint32_t)(r % oy) * 8u, z0 = (uint32_t)(r / oy) * 8u;
+    const uint32_t y1 = min(y0 + 8u, ny), z1 = min(z0 + 8u, nz);
+    for (uint32_t b = lane; b < ox; b += 32u) {
+      uint32_t m = 0;
+      for (uint32_t z = z0; z < z1; z++)
+#pragma unroll 8
+        for (uint32_t y = y0; y < y1; y++) {
+          const uint2 w = load8<VEC>(vox + ((size_t)z * ny + y) * nx, 8u * b, nx);
+          m = __vmaxu4(m, __vmaxu4(w.x, w.y));
+        }
+      raw[r * ox + b] = (uint8_t)max_byte(m);
+    }
+  }
+}
+
+cudaError_t launch_occ_raw(const uint8_t *vox, uint32_t nx, uint32_t ny, uint32_t nz, uint8_t *raw,
+                           cudaStream_t st) {
+  const uint32_t ox = (nx + 7u) / 8u, oy = (ny + 7u) / 8u, oz = (nz + 7u) / 8u;
+  if (nx % 8u == 0u && ((uintptr_t)vox & 7u) == 0u)
+    k_occ_raw<true><<<row_blocks((uint64_t)oy * oz), 256, 0, st>>>(vox, nx, ny, nz, raw, ox, oy, oz);
+  else
+    k_occ_raw<false><<<row_blocks((uint64_t)oy * oz), 256, 0, st>>>(vox, nx, ny, nz, raw, ox, oy, oz);
+  return cudaGetLastError();
+}
+
+// Quad words of a level: bound by the 4 bytes written per texel.
+__global__ void __launch_bounds__(256) k_level_quads(const uint8_t *__restrict__ src, uint32_t dx,
+                                                     uint32_t dy, uint32_t dz,
+                                                     uint32_t *__restrict__ quad) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint64_t rows = (uint64_t)dy * dz;
+  for (uint64_t r = blockIdx.x * 8ull + (threadIdx.x >> 5); r < rows; r += gridDim.x * 8ull) {
+    const uint8_t *row = src + r * dx, *next = r % dy + 1u < dy ? row + dx : row;
+    for (uint32_t x = lane * 4u; x < dx; x += 128u) {
+      // the row's bytes x .. x + 3 and, clamped, x + 4
+      uint32_t a = load4<false>(row, x, dx), b = load4<false>(next, x, dx);
+      const uint32_t left = dx - x;
+      if (left < 4u) {  // the last texel's neighbour is itself
+        a |= (a >> (8u * (left - 1u)) & 0xFFu) << (8u * left);
+        b |= (b >> (8u * (left - 1u)) & 0xFFu) << (8u * left);
+      }
+      const uint32_t an = left > 4u ? row[x + 4u] : a >> 24, bn = left > 4u ? next[x + 4u] : b >> 24;
+      const uint32_t alo = __byte_perm(a, 0u, 0x2110), ahi = __byte_perm(a, an, 0x4332);
+      const uint32_t blo = __byte_perm(b, 0u, 0x2110), bhi = __byte_perm(b, bn, 0x4332);
+      const uint32_t q[4] = {__byte_perm(alo, blo, 0x5410), __byte_perm(alo, blo, 0x7632),
+                             __byte_perm(ahi, bhi, 0x5410), __byte_perm(ahi, bhi, 0x7632)};
+      uint32_t *o = quad + r * dx + x;
+      if (!(dx & 3u)) {
+        *reinterpret_cast<uint4 *>(o) = make_uint4(q[0], q[1], q[2], q[3]);
+      } else {
+#pragma unroll
+        for (uint32_t k = 0; k < 4u; k++)
+          if (k < left) o[k] = q[k];
+      }
+    }
+  }
+}
+
+cudaError_t launch_level_quads(const uint8_t *src, uint32_t dx, uint32_t dy, uint32_t dz,
+                               uint32_t *quad, cudaStream_t st) {
+  k_level_quads<<<row_blocks((uint64_t)dy * dz), 256, 0, st>>>(src, dx, dy, dz, quad);
+  return cudaGetLastError();
+}
+
+size_t cube_quad_bytes(DevCube &c) {
+  if ((uint64_t)c.dim[0][0] * c.dim[0][1] * c.dim[0][2] > kQuadVoxels) return 0;
+  size_t words = 0;
+  for (uint32_t m = 0; m < c.nlevels; m++) {
+    c.qoff[m] = (uint32_t)words;
+    words += ((size_t)c.dim[m][0] * c.dim[m][1] * c.dim[m][2] + 63u) & ~(size_t)63u;
+  }
+  return words * sizeof(uint32_t);
+}
+
+cudaError_t build_cube_quads(DevCube &c, uint32_t *at, cudaStream_t st) {
+  c.quad = at;
+  cudaError_t e = cudaSuccess;
+  for (uint32_t m = 0; m < c.nlevels && at && e == cudaSuccess; m++)
+    e = launch_level_quads(c.lev[m], c.dim[m][0], c.dim[m][1], c.dim[m][2], at + c.qoff[m], st);
+  return e;
+}
+
 }  // namespace r3d

@@ -87,6 +87,21 @@ cudaError_t launch_level_down(const uint8_t *src, uint32_t sx, uint32_t sy, uint
 cudaError_t launch_slot_fill(const LevelSrc *lev, uint32_t nlev, const uint32_t *brick,
                              const uint32_t *slot, uint32_t njobs, uint8_t *pool, uint32_t *quad,
                              uint8_t *bmax, cudaStream_t st);
+// The cube's and the shard atlas's tables, of levels of any extent (x
+// fastest, no padding): the next mip (clamped source coordinates, (sum + 4) /
+// 8), the maxima of 8^3 blocks, and the quad words of DevCube::quad.
+cudaError_t launch_mip(const uint8_t *src, uint32_t sx, uint32_t sy, uint32_t sz, uint8_t *dst,
+                       uint32_t dx, uint32_t dy, uint32_t dz, cudaStream_t st);
+cudaError_t launch_occ_raw(const uint8_t *vox, uint32_t nx, uint32_t ny, uint32_t nz, uint8_t *raw,
+                           cudaStream_t st);
+cudaError_t launch_level_quads(const uint8_t *src, uint32_t dx, uint32_t dy, uint32_t dz,
+                               uint32_t *quad, cudaStream_t st);
+// Bytes of the quad words of a cube whose extents are set (0 past
+// kQuadVoxels), setting c.qoff; and the words themselves, at `at` (null:
+// none, the bytes are sampled), setting c.quad.
+size_t cube_quad_bytes(DevCube &c);
+cudaError_t build_cube_quads(DevCube &c, uint32_t *at, cudaStream_t st);
+
 // Quad words and block maxima of slots slot[0..njobs) (null: 0..njobs) of a
 // pool; the source slots may be another pool than the tables' (same index).
 cudaError_t launch_slot_tables(const uint8_t *pool, const uint32_t *slot, uint32_t njobs,

@@ -47,42 +47,6 @@ bool readable_in_place(const r3d_cuda_ctx *c, const void *p) {
 
 // ------------------------------------------------------------- builders
 
-// 2x box reduction with clamped source coordinates: (sum + 4) / 8
-__global__ void k_downsample_clamp(const uint8_t *__restrict__ src, uint32_t sx, uint32_t sy,
-                                   uint32_t sz, uint8_t *__restrict__ dst, uint32_t dx,
-                                   uint32_t dy, uint32_t dz) {
-  size_t n = (size_t)dx * dy * dz;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    uint32_t x = (uint32_t)(i % dx), y = (uint32_t)((i / dx) % dy), z = (uint32_t)(i / dx / dy);
-    uint32_t sum = 4u;
-#pragma unroll
-    for (uint32_t k = 0; k < 8u; k++) {
-      uint32_t xx = min(2u * x + (k & 1u), sx - 1u), yy = min(2u * y + ((k >> 1) & 1u), sy - 1u),
-               zz = min(2u * z + (k >> 2), sz - 1u);
-      sum += src[((size_t)zz * sy + yy) * sx + xx];
-    }
-    dst[i] = (uint8_t)(sum >> 3);
-  }
-}
-
-// 8^3 block maxima (src/vk/vkbackend.c:794-824)
-__global__ void k_occ_raw(const uint8_t *__restrict__ vox, uint32_t nx, uint32_t ny, uint32_t nz,
-                          uint8_t *__restrict__ raw, uint32_t ox, uint32_t oy, uint32_t oz) {
-  size_t n = (size_t)ox * oy * oz;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    uint32_t bx = (uint32_t)(i % ox), by = (uint32_t)((i / ox) % oy), bz = (uint32_t)(i / ox / oy);
-    uint32_t m = 0;
-    for (uint32_t z = bz * 8u; z < min(bz * 8u + 8u, nz); z++)
-      for (uint32_t y = by * 8u; y < min(by * 8u + 8u, ny); y++) {
-        const uint8_t *row = vox + ((size_t)z * ny + y) * nx;
-        for (uint32_t x = bx * 8u; x < min(bx * 8u + 8u, nx); x++) m = max(m, (uint32_t)row[x]);
-      }
-    raw[i] = (uint8_t)m;
-  }
-}
-
 // 26-neighbour max dilation (src/vk/vkbackend.c:845-860)
 __global__ void k_occ_dilate(const uint8_t *__restrict__ raw, uint8_t *__restrict__ dil,
                              uint32_t ox, uint32_t oy, uint32_t oz) {
@@ -101,6 +65,18 @@ __global__ void k_occ_dilate(const uint8_t *__restrict__ raw, uint8_t *__restric
         }
     dil[i] = (uint8_t)m;
   }
+}
+
+
+template <class T>
+static cudaError_t reserve(T *&p, size_t &cap, size_t need) {
+  if (keeps(p, cap, need)) return cudaDeviceSynchronize();
+  cudaFree(p);
+  p = nullptr;
+  cap = 0;
+  const cudaError_t e = cudaMalloc(&p, need);
+  if (e == cudaSuccess) cap = need;
+  return e;
 }
 
 static unsigned grid_for(size_t n) {
@@ -185,6 +161,8 @@ void r3d_cuda_destroy(r3d_cuda_ctx *c) {
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
   cudaFree(c->cube_buf);
+  cudaFree(c->cube_quad);
+  cudaFree(c->shard_quad);
   cudaFree(c->page);
   cudaFree(c->pool);
   cudaFree(c->bmax);
@@ -263,33 +241,56 @@ int r3d_cuda_upload_volume(r3d_cuda_ctx *c, const r3d_volume_desc *d, const uint
   size_t total = off[mips] + ((onb + 255) & ~(size_t)255);
   uint8_t *buf = nullptr, *raw = nullptr;
   R3D_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-  cudaError_t e = cudaMalloc(&buf, total + onb);
+  // bytes, occupancy (and its raw grid) and quad words in one allocation,
+  // kept when about this size as the brick cache's are; the words stand alone
+  // when the whole does not fit beside the volume it replaces
+  const size_t base = (total + onb + 255) & ~(size_t)255, qbytes = cube_quad_bytes(cube);
+  const bool kept = keeps(c->cube_buf, c->cube_cap, base + qbytes);
+  bool whole = true;
+  cudaError_t e = kept ? cudaDeviceSynchronize() : cudaMalloc(&buf, base + qbytes);
+  if (e == cudaErrorMemoryAllocation && qbytes) {
+    cudaGetLastError();
+    whole = false;
+    e = cudaMalloc(&buf, base);
+  }
   if (e != cudaSuccess) return cuda_fail(c, e, "upload_volume: cudaMalloc");
+  if (kept) {
+    buf = c->cube_buf;
+    c->have_cube = false;
+  }
   raw = buf + total;
   e = cudaMemcpyAsync(buf, voxels, (size_t)nx * ny * nz, cudaMemcpyDefault, c->stream);
-  for (uint32_t m = 1; m < mips && e == cudaSuccess; m++) {
-    size_t n = (size_t)cube.dim[m][0] * cube.dim[m][1] * cube.dim[m][2];
-    k_downsample_clamp<<<grid_for(n), 256, 0, c->stream>>>(
-        buf + off[m - 1], cube.dim[m - 1][0], cube.dim[m - 1][1], cube.dim[m - 1][2], buf + off[m],
-        cube.dim[m][0], cube.dim[m][1], cube.dim[m][2]);
-    e = cudaGetLastError();
-  }
+  for (uint32_t m = 0; m < mips; m++) cube.lev[m] = buf + off[m];
+  cube.occ = buf + off[mips];
+  for (uint32_t m = 1; m < mips && e == cudaSuccess; m++)
+    e = launch_mip(cube.lev[m - 1], cube.dim[m - 1][0], cube.dim[m - 1][1], cube.dim[m - 1][2],
+                   buf + off[m], cube.dim[m][0], cube.dim[m][1], cube.dim[m][2], c->stream);
+  if (e == cudaSuccess) e = launch_occ_raw(buf, nx, ny, nz, raw, c->stream);
   if (e == cudaSuccess) {
-    k_occ_raw<<<grid_for(onb), 256, 0, c->stream>>>(buf, nx, ny, nz, raw, cube.odim[0],
-                                                    cube.odim[1], cube.odim[2]);
     k_occ_dilate<<<grid_for(onb), 256, 0, c->stream>>>(raw, buf + off[mips], cube.odim[0],
                                                        cube.odim[1], cube.odim[2]);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) {
-    cudaFree(buf);
+    if (!kept) cudaFree(buf);
     return cuda_fail(c, e, "upload_volume");
   }
-  for (uint32_t m = 0; m < mips; m++) cube.lev[m] = buf + off[m];
-  cube.occ = buf + off[mips];
-  cudaFree(c->cube_buf);
-  c->cube_buf = buf;
+  if (!kept) {
+    cudaFree(c->cube_buf);
+    c->cube_buf = buf;
+    c->cube_cap = whole ? base + qbytes : base;
+  }
+  c->have_cube = false;
+  c->cube.quad = nullptr;
+  cudaFree(c->cube_quad);
+  c->cube_quad = nullptr;
+  uint32_t *words = whole && qbytes ? (uint32_t *)(buf + base) : nullptr;
+  if (!whole && cudaMalloc(&c->cube_quad, qbytes) == cudaSuccess) words = c->cube_quad;
+  if (!whole) cudaGetLastError();
+  e = build_cube_quads(cube, words, c->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  if (e != cudaSuccess) return cuda_fail(c, e, "upload_volume: quad words");
   c->cube_bytes = total;
   c->have_cube = true;
   c->cube = cube;
@@ -368,25 +369,6 @@ static int decode_header(r3d_cuda_ctx *c, const uint32_t *page, uint32_t words, 
   b.page_words = words;
   b.nslots = nslots;
   return R3D_OK;
-}
-
-// Device buffers of a brick cache outlive a rebuild of about the same size:
-// one of at least `need` and less than twice that many bytes is used again
-// (a 1024^3 cache's cudaMalloc and cudaFree calls took 10 ms of a rebuild's
-// 23), any other is replaced.  Frames in flight on other streams may still
-// read a kept buffer, so the device is idle before it is written again, as
-// cudaFree leaves it too.
-static bool keeps(const void *p, size_t cap, size_t need) { return p && cap >= need && need > cap / 2; }
-
-template <class T>
-static cudaError_t reserve(T *&p, size_t &cap, size_t need) {
-  if (keeps(p, cap, need)) return cudaDeviceSynchronize();
-  cudaFree(p);
-  p = nullptr;
-  cap = 0;
-  const cudaError_t e = cudaMalloc(&p, need);
-  if (e == cudaSuccess) cap = need;
-  return e;
 }
 
 // Room for the per-slot tables (block maxima, quad words) of c->nslots

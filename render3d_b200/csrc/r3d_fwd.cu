@@ -12,7 +12,7 @@
 // or parked shading, not the step heatmap) get one block more, MIP two, all
 // without spills: 1080p FULL runs 2 % faster at 64 registers and MIP 5 %
 // at 56, while the overlay and shard kernels lose 14 % and 4 % and the
-// heatmap 3 % at 8 blocks, and FULL spills at 9.
+// heatmap 3 % at 8 blocks, and FULL spills at 9.  The quad paths: kQuadBlocks.
 #ifndef R3D_FWD_MIN_BLOCKS
 #define R3D_FWD_MIN_BLOCKS 7
 #endif
@@ -23,7 +23,7 @@
 #if R3D_FWD_MIN_BLOCKS > 0
 #define R3D_FWD_BOUNDS                                                                     \
   __launch_bounds__(R3D_FWD_WARPS * 32,                                                    \
-                    (R3D_FWD_MIN_BLOCKS + (PATH == PATH_LOD_BRICKS && !OVL && !COUNT &&    \
+                    (kQuadPath<PATH> ? kQuadBlocks<PATH>(QUEUE) : R3D_FWD_MIN_BLOCKS + (PATH == PATH_LOD_BRICKS && !OVL && !COUNT &&    \
                                                    !QUEUE && MODE != R3D_MODE_HEATMAP            \
                                                ? (MODE == R3D_MODE_MIP ? 2 : 1)                  \
                                                : 0)) * 4 / R3D_FWD_WARPS)
@@ -73,7 +73,7 @@ __global__ void R3D_FWD_BOUNDS k_raycast(const __grid_constant__ r3d_frame_param
   constexpr uint32_t kStrip = PATH == PATH_LOD_BRICKS && MODE == R3D_MODE_MIP ? 32u : 0u;
   constexpr bool kMidRows =
       kFwdWarps == 4u && (MODE == R3D_MODE_FULL || MODE == R3D_MODE_FLAT) &&
-      (PATH == PATH_LOD_BRICKS || PATH == PATH_SHARD || PATH == PATH_CUBE);
+      (PATH == PATH_LOD_BRICKS || PATH == PATH_CUBE || kShardPath<PATH> || kQuadPath<PATH>);
   uint32_t bx = blockIdx.x, by = blockIdx.y;
   if (kStrip) {
     const uint32_t nby = gridDim.y, lin = blockIdx.y * gridDim.x + blockIdx.x;
@@ -225,7 +225,7 @@ static cudaError_t launch_p(const r3d_frame_params &pc, const DevScene &s, bool 
 }
 
 #ifdef R3D_FWD_PATH
-// The build compiles this file once per sampling path (R3D_FWD_PATH = 0..5)
+// The build compiles this file once per sampling path (R3D_FWD_PATH = 0..7)
 // so that the paths' kernels compile in parallel; each object defines its
 // path's entry.
 template <>
@@ -261,7 +261,7 @@ cudaError_t launch_view(const r3d_cuda_ctx *c, const r3d_frame_params &pc, uint8
   DevScene s = c->scene();
   s.el = elide_counts(pc, s.tf_zero_t);
   const bool fast = c->quality == R3D_QUALITY_FAST;
-  const int path = path_of_view(pc);
+  const int path = quad_path(path_of_view(pc), &s, 1u);
   const uint32_t shade = c->sched.shade_group;  // 0: the path's default (kShadeQueued)
 #define R3D_PATH_CASE(P)                                                                   \
   case P:                                                                                  \
@@ -273,6 +273,8 @@ cudaError_t launch_view(const r3d_cuda_ctx *c, const r3d_frame_params &pc, uint8
     R3D_PATH_CASE(PATH_SLAB);
     R3D_PATH_CASE(PATH_LOD_BRICKS);
     R3D_PATH_CASE(PATH_SHARD);
+    R3D_PATH_CASE(PATH_SHARD_QUAD);
+    R3D_PATH_CASE(PATH_CUBE_QUAD);
     default:
       return launch_path<PATH_CUBE>(pc, s, fast, c->lut, img, out_w, steps, mip_index, total,
                                     counters, shade, rows, stream);

@@ -17,7 +17,8 @@ struct r3d_cuda_ctx {
 
   // cube volume: all mip levels in one allocation, then the occupancy grid
   uint8_t *cube_buf = nullptr;
-  size_t cube_bytes = 0;
+  size_t cube_bytes = 0, cube_cap = 0;
+  uint32_t *cube_quad = nullptr;  // the cube's quad words when not in cube_buf
   bool have_cube = false;
   r3d::DevCube cube{};
 
@@ -121,6 +122,8 @@ struct r3d_cuda_ctx {
   // single-level brick atlas: 4 mip levels, then the world-indexed
   // occupancy grid, in one allocation; page table of bpa^3 entries
   uint8_t *shard_buf = nullptr;
+  size_t shard_cap = 0;
+  uint32_t *shard_quad = nullptr;  // the atlas's quad words when not in shard_buf
   uint32_t *shard_page = nullptr;
   bool have_shard = false;
   r3d::DevShard sh{};
@@ -183,6 +186,16 @@ struct r3d_cuda_ctx {
 };
 
 namespace r3d {
+
+// A volume's device buffers outlive a rebuild of about the same size:
+// one of at least `need` and less than twice that many bytes is used again
+// (a 1024^3 brick cache's cudaMalloc and cudaFree calls took 10 ms of a rebuild's
+// 23), any other is replaced.  Frames in flight on other streams may still
+// read a kept buffer, so the device is idle before it is written again, as
+// cudaFree leaves it too.
+inline bool keeps(const void *p, size_t cap, size_t need) {
+  return p && cap >= need && need > cap / 2;
+}
 
 int fail(r3d_cuda_ctx *c, int code, const char *fmt, ...);
 int cuda_fail(r3d_cuda_ctx *c, cudaError_t e, const char *what);

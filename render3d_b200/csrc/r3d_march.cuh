@@ -29,9 +29,27 @@ enum Path {
   PATH_SHARD = 2,
   PATH_SLAB = 3,
   PATH_CLIP = 4,
-  PATH_VSLAB = 5
+  PATH_VSLAB = 5,
+  // the cube and the shard atlas read through quad words (DevCube::quad); a
+  // launch takes them in place of PATH_CUBE / PATH_SHARD when its scenes
+  // hold the words (quad_path)
+  PATH_CUBE_QUAD = 6,
+  PATH_SHARD_QUAD = 7
 };
-constexpr int kNumPaths = 6;
+template <int PATH>
+constexpr bool kQuadPath = PATH == PATH_CUBE_QUAD || PATH == PATH_SHARD_QUAD;
+// 128-thread blocks per SM that the kernels of the quad paths leave registers
+// for.  Their marches wait on memory with the SMs far from full (the long
+// rays of a view end last), so FULL, whose shading spills 60-212 bytes at 7
+// blocks, runs fastest with 4 (512^3 shard frame 1.37 -> 0.99 ms, 256^3 cube
+// 0.384 -> 0.321, thumbnail 0.146 -> 0.129; 5 blocks 1.00, 0.338, 0.135; 3
+// blocks 1.04, 0.315, 0.127), the shard's other modes with 5 (MIP 1.33 -> 1.19).
+template <int PATH>
+constexpr int kQuadBlocks(bool full) {
+  return full ? 4 : PATH == PATH_SHARD_QUAD ? 5 : 7;
+}
+template <int PATH>
+constexpr bool kShardPath = PATH == PATH_SHARD || PATH == PATH_SHARD_QUAD;
 // slab_grid bit of a virtual-slab view (vkbackend.c:6629); a tiled slab's
 // slab_grid stops at bit 23 (its overview scale, at most 32, in bits 16..23)
 constexpr uint32_t kVslabGrid = 1u << 24;
@@ -57,7 +75,16 @@ struct DevCube {
   uint32_t maxdim;
   const uint8_t *occ;
   uint32_t odim[3];
+  // per texel of level m, from word qoff[m]: the bytes at (x, y), (x1, y),
+  // (x, y1), (x1, y1) of its z plane, x1 = min(x + 1, dim - 1) and y1
+  // likewise; nullptr when the volume is too large for them (kQuadVoxels) or
+  // they did not fit the memory
+  const uint32_t *quad;
+  uint32_t qoff[kMaxLevels];
 };
+// Level-0 voxels up to which a cube or atlas gets quad words: 32-bit word
+// indices over all levels, and at most 10 GB beside 2.4 GB of bytes.
+constexpr uint64_t kQuadVoxels = 1ull << 31;
 
 // LOD brick cache.  The page-table header is validated and decoded on the
 // host when the cache is loaded; entries are read from device memory.
@@ -230,6 +257,18 @@ struct DevScene {
   ElideCounts el;
 };
 
+// The path a launch over scenes s[0, n) samples `path` through: the quad
+// words' when every scene that has the volume holds them.  Decided from the
+// launched scenes themselves, since a plan outlives an upload.
+inline int quad_path(int path, const DevScene *s, uint32_t n) {
+  if (path != PATH_CUBE && path != PATH_SHARD) return path;
+  for (uint32_t k = 0; k < n; k++) {
+    const DevCube &c = path == PATH_CUBE ? s[k].cube : s[k].sh.atlas;
+    if (c.lev[0] && !c.quad) return path;
+  }
+  return path == PATH_CUBE ? PATH_CUBE_QUAD : PATH_SHARD_QUAD;
+}
+
 struct RayResult {
   float rgb[3];
   uint32_t steps;
@@ -284,60 +323,124 @@ __device__ __forceinline__ float lerp_raw(float ra, float rb, float t) {
   return fmaf(t, rb - ra, ra - 8388608.0f);
 }
 
-// Clamp-to-edge trilinear at texel centres on a u8 grid: x, then y, then z
-// lerps in 0..255 space, scaled by 1/255 at the end.
-__device__ __forceinline__ float tri_u8(const uint8_t *__restrict__ g, uint32_t dx, uint32_t dy,
-                                        uint32_t dz, float tx, float ty, float tz) {
-  tx = clamp_(tx, 0.0f, (float)(dx - 1u));
-  ty = clamp_(ty, 0.0f, (float)(dy - 1u));
-  tz = clamp_(tz, 0.0f, (float)(dz - 1u));
-  float fx, fy, fz;
-  const uint32_t x0 = floor_frac(tx, fx), y0 = floor_frac(ty, fy), z0 = floor_frac(tz, fz);
-  uint32_t x1 = min(x0 + 1u, dx - 1u), y1 = min(y0 + 1u, dy - 1u), z1 = min(z0 + 1u, dz - 1u);
-  size_t sy = dx, sz = (size_t)dx * dy;
-  const uint8_t *r00 = g + (size_t)y0 * sy + (size_t)z0 * sz;
-  const uint8_t *r10 = g + (size_t)y1 * sy + (size_t)z0 * sz;
-  const uint8_t *r01 = g + (size_t)y0 * sy + (size_t)z1 * sz;
-  const uint8_t *r11 = g + (size_t)y1 * sy + (size_t)z1 * sz;
-  float c00 = lerp_raw(raw_u8(r00 + x0), raw_u8(r00 + x1), fx);
-  float c10 = lerp_raw(raw_u8(r10 + x0), raw_u8(r10 + x1), fx);
-  float c01 = lerp_raw(raw_u8(r01 + x0), raw_u8(r01 + x1), fx);
-  float c11 = lerp_raw(raw_u8(r11 + x0), raw_u8(r11 + x1), fx);
-  float e0 = lerp_(c00, c10, fy), e1 = lerp_(c01, c11, fy);
-  return lerp_(e0, e1, fz) * kInv255;
+// byte k of w as the float 2^23 + byte (see lerp_raw)
+__device__ __forceinline__ float qraw(uint32_t w, uint32_t k) {
+  return __uint_as_float(__byte_perm(w, 0x4B000000u, k | 0x7540u));
+}
+
+// One axis of a clamp-to-edge trilinear lookup at texel centres: base texel
+// and fraction.  The axes of a position are independent, so the gradient taps
+// of a sample, which move one axis each, share the others.
+struct CubeAxis {
+  uint32_t i0;
+  float f;
+};
+__device__ __forceinline__ CubeAxis cube_axis(uint32_t n, float p) {
+  CubeAxis a;
+  a.i0 = floor_frac(clamp_(fmaf(p, (float)n, -0.5f), 0.0f, (float)(n - 1u)), a.f);
+  return a;
+}
+
+// The lookup in level m at three axes: x, then y, then z lerps in 0..255
+// space, scaled by 1/255 at the end.  QUAD: two words of the level's quad
+// grid; else its eight bytes (eight loads and their addresses per level: the
+// 256^3 cube's frame takes 0.56 ms with them and 0.34 with the words, the
+// 512^3 shard's 1.81 and 1.20, its MIP view 2.33 and 1.37).
+template <bool QUAD>
+__device__ __forceinline__ float cube_fetch(const DevCube &c, uint32_t m, const CubeAxis &x,
+                                            const CubeAxis &y, const CubeAxis &z) {
+  const uint32_t dx = c.dim[m][0], dy = c.dim[m][1], dz = c.dim[m][2];
+  float c00, c10, c01, c11;
+  if (QUAD) {
+    const uint32_t plane = dx * dy;
+    const uint32_t *r = c.quad + (c.qoff[m] + (z.i0 * plane + (y.i0 * dx + x.i0)));
+    const uint32_t w0 = __ldg(r), w1 = __ldg(r + (z.i0 + 1u < dz ? plane : 0u));
+    c00 = lerp_raw(qraw(w0, 0), qraw(w0, 1), x.f);
+    c10 = lerp_raw(qraw(w0, 2), qraw(w0, 3), x.f);
+    c01 = lerp_raw(qraw(w1, 0), qraw(w1, 1), x.f);
+    c11 = lerp_raw(qraw(w1, 2), qraw(w1, 3), x.f);
+  } else {
+    const uint32_t x1 = min(x.i0 + 1u, dx - 1u), y1 = min(y.i0 + 1u, dy - 1u),
+                   z1 = min(z.i0 + 1u, dz - 1u);
+    const size_t sy = dx, sz = (size_t)dx * dy;
+    const uint8_t *g = c.lev[m];
+    const uint8_t *r00 = g + (size_t)y.i0 * sy + (size_t)z.i0 * sz;
+    const uint8_t *r10 = g + (size_t)y1 * sy + (size_t)z.i0 * sz;
+    const uint8_t *r01 = g + (size_t)y.i0 * sy + (size_t)z1 * sz;
+    const uint8_t *r11 = g + (size_t)y1 * sy + (size_t)z1 * sz;
+    c00 = lerp_raw(raw_u8(r00 + x.i0), raw_u8(r00 + x1), x.f);
+    c10 = lerp_raw(raw_u8(r10 + x.i0), raw_u8(r10 + x1), x.f);
+    c01 = lerp_raw(raw_u8(r01 + x.i0), raw_u8(r01 + x1), x.f);
+    c11 = lerp_raw(raw_u8(r11 + x.i0), raw_u8(r11 + x1), x.f);
+  }
+  return lerp_(lerp_(c00, c10, y.f), lerp_(c01, c11, y.f), z.f) * kInv255;
+}
+
+// The levels of a lookup at lod: floor(lod) and, when fr > 0, the next.
+struct CubeLevels {
+  uint32_t m;
+  float fr;  // 0: one level
+};
+__device__ __forceinline__ CubeLevels cube_levels(const DevCube &c, float lod) {
+  const float fl = floorf(lod);
+  CubeLevels l;
+  l.m = min((uint32_t)fl, c.nlevels - 1u);
+  l.fr = l.m + 1u < c.nlevels ? lod - fl : 0.0f;
+  return l;
+}
+
+template <bool QUAD>
+__device__ __forceinline__ float cube_level_sample(const DevCube &c, uint32_t m, float3 p) {
+  return cube_fetch<QUAD>(c, m, cube_axis(c.dim[m][0], p.x), cube_axis(c.dim[m][1], p.y),
+                          cube_axis(c.dim[m][2], p.z));
 }
 
 // volumes[0].SampleLevel(p, lod): trilinear within a level, linear between
 // floor(lod) and floor(lod)+1 (raycast.slang:409-416, vkbackend.c:1058-1069)
+template <bool QUAD>
 __device__ __forceinline__ float cube_sample(const DevCube &c, float3 p, float lod) {
-  float fl = floorf(lod);
-  uint32_t m0 = min((uint32_t)fl, c.nlevels - 1u);
-  float fr = lod - fl;
-  float v = tri_u8(c.lev[m0], c.dim[m0][0], c.dim[m0][1], c.dim[m0][2],
-                   fmaf(p.x, (float)c.dim[m0][0], -0.5f), fmaf(p.y, (float)c.dim[m0][1], -0.5f),
-                   fmaf(p.z, (float)c.dim[m0][2], -0.5f));
-  if (fr > 0.0f && m0 + 1u < c.nlevels) {
-    uint32_t m1 = m0 + 1u;
-    float v1 = tri_u8(c.lev[m1], c.dim[m1][0], c.dim[m1][1], c.dim[m1][2],
-                      fmaf(p.x, (float)c.dim[m1][0], -0.5f),
-                      fmaf(p.y, (float)c.dim[m1][1], -0.5f),
-                      fmaf(p.z, (float)c.dim[m1][2], -0.5f));
-    v = lerp_(v, v1, fr);
-  }
+  const CubeLevels l = cube_levels(c, lod);
+  float v = cube_level_sample<QUAD>(c, l.m, p);
+  if (l.fr > 0.0f) v = lerp_(v, cube_level_sample<QUAD>(c, l.m + 1u, p), l.fr);
   return v;
 }
 
-// occ.SampleLevel(p, 0) with a nearest sampler
-__device__ __forceinline__ float occ_sample(const DevCube &c, float3 p) {
-  float q[3] = {floorf(p.x * (float)c.odim[0]), floorf(p.y * (float)c.odim[1]),
-                floorf(p.z * (float)c.odim[2])};
-  uint32_t i[3];
-#pragma unroll
-  for (int a = 0; a < 3; a++) {
-    float m = (float)(c.odim[a] - 1u);
-    i[a] = !(q[a] >= 0.0f) ? 0u : (q[a] > m ? c.odim[a] - 1u : (uint32_t)q[a]);
-  }
-  return (float)__ldg(c.occ + ((size_t)i[2] * c.odim[1] + i[1]) * c.odim[0] + i[0]) * kInv255;
+// The samples at p +- e along each axis (+x, -x, +y, -y, +z, -z) of level m.
+template <bool QUAD>
+__device__ __forceinline__ void cube_taps6(const DevCube &c, uint32_t m, float3 p, float e,
+                                           float (&v)[6]) {
+  const uint32_t *n = c.dim[m];
+  const CubeAxis x = cube_axis(n[0], p.x), y = cube_axis(n[1], p.y), z = cube_axis(n[2], p.z);
+  v[0] = cube_fetch<QUAD>(c, m, cube_axis(n[0], p.x + e), y, z);
+  v[1] = cube_fetch<QUAD>(c, m, cube_axis(n[0], p.x - e), y, z);
+  v[2] = cube_fetch<QUAD>(c, m, x, cube_axis(n[1], p.y + e), z);
+  v[3] = cube_fetch<QUAD>(c, m, x, cube_axis(n[1], p.y - e), z);
+  v[4] = cube_fetch<QUAD>(c, m, x, y, cube_axis(n[2], p.z + e));
+  v[5] = cube_fetch<QUAD>(c, m, x, y, cube_axis(n[2], p.z - e));
+}
+// The samples at p + e (+--), (--+), (-+-), (+++) of level m.
+template <bool QUAD>
+__device__ __forceinline__ void cube_taps4(const DevCube &c, uint32_t m, float3 p, float e,
+                                           float (&v)[4]) {
+  const uint32_t *n = c.dim[m];
+  const CubeAxis xp = cube_axis(n[0], p.x + e), xm = cube_axis(n[0], p.x - e);
+  const CubeAxis yp = cube_axis(n[1], p.y + e), ym = cube_axis(n[1], p.y - e);
+  const CubeAxis zp = cube_axis(n[2], p.z + e), zm = cube_axis(n[2], p.z - e);
+  v[0] = cube_fetch<QUAD>(c, m, xp, ym, zm);
+  v[1] = cube_fetch<QUAD>(c, m, xm, ym, zp);
+  v[2] = cube_fetch<QUAD>(c, m, xm, yp, zm);
+  v[3] = cube_fetch<QUAD>(c, m, xp, yp, zp);
+}
+
+// occ.SampleLevel(p, 0) with a nearest sampler: the occupancy byte under p.
+// (Clamping before the floor gives the same cell: a position below the grid,
+// or NaN, its first, one past it its last.)
+__device__ __forceinline__ uint32_t occ_byte(const DevCube &c, float3 p) {
+  float f;
+  const uint32_t x = floor_frac(clamp_(p.x * (float)c.odim[0], 0.0f, (float)(c.odim[0] - 1u)), f);
+  const uint32_t y = floor_frac(clamp_(p.y * (float)c.odim[1], 0.0f, (float)(c.odim[1] - 1u)), f);
+  const uint32_t z = floor_frac(clamp_(p.z * (float)c.odim[2], 0.0f, (float)(c.odim[2] - 1u)), f);
+  return __ldg(c.occ + ((size_t)z * c.odim[1] + y) * c.odim[0] + x);
 }
 
 struct BrickCtx {  // raycast.slang:144-152
@@ -494,9 +597,6 @@ __device__ __forceinline__ float qbyte(uint32_t w, uint32_t k) {
 // in 0..255 space, x then y then z, as on the byte grid.
 // The trilinear value of the quad words w0 (plane z0) and w1 (plane z1).
 // The x lerps take the bytes as 2^23 + byte (the permute alone; lerp_raw).
-__device__ __forceinline__ float qraw(uint32_t w, uint32_t k) {
-  return __uint_as_float(__byte_perm(w, 0x4B000000u, k | 0x7540u));
-}
 // The eight bytes of two quad words, as 2^23 + byte.
 struct RawBytes {
   float r[8];
@@ -617,13 +717,14 @@ __device__ __forceinline__ float3 shard_slot_org(const DevShard &h, uint32_t slo
 // brick-local position clamped to [inset, 128 - inset] with
 // inset = max(0.5 * 2^lod, 0.5), then the atlas sampled at lod like a cube
 // texture.  e2 = r3d_exp2f(lod).
+template <bool QUAD>
 __device__ __forceinline__ float shard_fetch(const DevShard &h, float3 org, float3 bl, float lod,
                                              float e2) {
   const float inset = fmaxf(0.5f * e2, 0.5f), hi = 128.0f - inset;
   const float3 u = make_float3((org.x + clamp_(bl.x, inset, hi)) * h.inv_adim,
                                (org.y + clamp_(bl.y, inset, hi)) * h.inv_adim,
                                (org.z + clamp_(bl.z, inset, hi)) * h.inv_adim);
-  return cube_sample(h.atlas, u, lod);
+  return cube_sample<QUAD>(h.atlas, u, lod);
 }
 
 // The lookups of the section paths (tiled slab, virtual slab, clipmap) are
@@ -873,7 +974,7 @@ __device__ __forceinline__ float byte_float(uint32_t m) {
 
 // Per-view constants of the march (raycast.slang:647-683,722-762).
 struct ViewConst {
-  float voxel, vox_inv, max_lod, cone, dt, bs, occ_gate, bgate, opac_k;
+  float voxel, vox_inv, max_lod, cone, dt, bs, rbs, occ_gate, bgate, opac_k;
   float lod_bias, threshold, density;
   float3 ext;
   bool ortho, lod_on;
@@ -895,7 +996,7 @@ __device__ __forceinline__ ViewConst view_const(const r3d_frame_params &pc, cons
     v.vox_inv = s.br.md;
     v.max_lod = (float)(s.br.nlev - 1u);
     v.ext = make_float3(s.br.bs[0] / s.br.md, s.br.bs[1] / s.br.md, s.br.bs[2] / s.br.md);
-  } else if (PATH == PATH_SHARD) {  // raycast.slang:659-661: the atlas has 4 mips
+  } else if (kShardPath<PATH>) {  // raycast.slang:659-661: the atlas has 4 mips
     v.voxel = 1.0f / s.sh.n;
     v.vox_inv = s.sh.n;
     v.max_lod = 3.0f;
@@ -930,6 +1031,7 @@ __device__ __forceinline__ ViewConst view_const(const r3d_frame_params &pc, cons
   v.cone = (2.0f * sqrtf(dot3(up, up))) / (float)pc.viewport[1];
   v.dt = pc.step_voxels * v.voxel;
   v.bs = 8.0f * v.voxel;
+  v.rbs = 1.0f / v.bs;
   v.occ_gate = fmaxf(pc.skip_gate, 0.5f / 255.0f);
   v.bgate = fmaxf(v.occ_gate, 4.5f / 255.0f);
   v.opac_k = pc.density * pc.step_voxels;
@@ -974,6 +1076,7 @@ struct Pending {
 // State of one ray between march steps.
 struct RayState {
   float3 ro, dir;  // volume space
+  float rdir[3];   // 1 / dir (cube and shard paths)
   float t, tf_, span_step;
   bool span_dom;  // span_step >= every exp2(lod): lod_step is span_step
   // LOD bricks: for t in [lod_tlo, lod_thi) the desired level is
@@ -1076,6 +1179,7 @@ __device__ __forceinline__ bool ray_begin(const r3d_frame_params &pc, const DevS
 #pragma unroll
   for (int a = 0; a < 3; a++) {
     float inv = 1.0f / dv[a];
+    st.rdir[a] = inv;
     float t0 = (lo[a] - ov[a]) * inv, t1 = (hi[a] - ov[a]) * inv;
     tmn[a] = fminf(t0, t1);
     tmx[a] = fmaxf(t0, t1);
@@ -1135,6 +1239,23 @@ __device__ __forceinline__ float skip_block(const RayState &st, float3 p, float 
   return fmaxf(fminf(fminf(tex[0], tex[1]), tex[2]), st.t) + bsz * 0.01f;
 }
 
+// The same jump with rbsz = 1 / bsz and the ray's reciprocal direction: on
+// the cube and shard paths most steps of a march are jumps, and their two
+// rounds of divisions stood on its critical path (r3d_div_rcp: the same
+// bits).  LOD bricks jump whole bricks, seldom, and have no registers left
+// for the reciprocals.
+__device__ __forceinline__ float skip_block(const RayState &st, float3 p, float bsz, float rbsz) {
+  float pv[3] = {p.x, p.y, p.z}, dv[3] = {st.dir.x, st.dir.y, st.dir.z},
+        ov[3] = {st.ro.x, st.ro.y, st.ro.z};
+  float tex[3];
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    float nextp = (floorf(r3d_div_rcp(pv[a], bsz, rbsz)) + (dv[a] > 0.0f ? 1.0f : 0.0f)) * bsz;
+    tex[a] = fabsf(dv[a]) > 1e-8f ? r3d_div_rcp(nextp - ov[a], dv[a], st.rdir[a]) : 1e30f;
+  }
+  return fmaxf(fminf(fminf(tex[0], tex[1]), tex[2]), st.t) + bsz * 0.01f;
+}
+
 // The level a section sample was looked up at: its taps read the same one
 // (clipmap: the level the sample picked; raycast.slang:942-946,967-974).
 template <int PATH>
@@ -1149,7 +1270,7 @@ template <int PATH, int MODE, bool FAST, bool OVL = false>
 __device__ __forceinline__ float3 sample_color(const DevScene &s, const ViewConst &vc, float3 dir,
                                                const Pending &q) {
   constexpr bool kLod = PATH == PATH_LOD_BRICKS;
-  constexpr bool kShard = PATH == PATH_SHARD;
+  constexpr bool kShard = kShardPath<PATH>, kQuad = kQuadPath<PATH>;
   constexpr bool kShaded = MODE == R3D_MODE_FULL;
   float col_r = q.sm.x, col_g = q.sm.y, col_b = q.sm.z;
   if (OVL && q.reg_live) {  // green/magenta fuse in TF space, before shading (:910-914)
@@ -1194,10 +1315,10 @@ __device__ __forceinline__ float3 sample_color(const DevScene &s, const ViewCons
         const float ev = q.lod_step * ir3;
         const float3 u = q.bl, org = shard_slot_org(s.sh, q.slot);
         const float e2 = r3d_exp2f(q.lod);
-        q0 = shard_fetch(s.sh, org, make_float3(u.x + ev, u.y - ev, u.z - ev), q.lod, e2);
-        q1 = shard_fetch(s.sh, org, make_float3(u.x - ev, u.y - ev, u.z + ev), q.lod, e2);
-        q2 = shard_fetch(s.sh, org, make_float3(u.x - ev, u.y + ev, u.z - ev), q.lod, e2);
-        q3 = shard_fetch(s.sh, org, make_float3(u.x + ev, u.y + ev, u.z + ev), q.lod, e2);
+        q0 = shard_fetch<kQuad>(s.sh, org, make_float3(u.x + ev, u.y - ev, u.z - ev), q.lod, e2);
+        q1 = shard_fetch<kQuad>(s.sh, org, make_float3(u.x - ev, u.y - ev, u.z + ev), q.lod, e2);
+        q2 = shard_fetch<kQuad>(s.sh, org, make_float3(u.x - ev, u.y + ev, u.z - ev), q.lod, e2);
+        q3 = shard_fetch<kQuad>(s.sh, org, make_float3(u.x + ev, u.y + ev, u.z + ev), q.lod, e2);
       } else if (kSection) {  // two values per axis: (+--), (--+), (-+-), (+++)
         const float ee = (vc.voxel * q.lod_step) * ir3;
         if (PATH == PATH_CLIP && (int)q.slot < 0) {  // no level at the sample: each tap its own
@@ -1216,11 +1337,17 @@ __device__ __forceinline__ float3 sample_color(const DevScene &s, const ViewCons
           q3 = sec_fetch<PATH>(s, L, xp, yp, zp);
         }
       } else {
-        float ee = (vc.voxel * q.lod_step) * ir3;
-        q0 = cube_sample(tex, make_float3(q.p.x + ee, q.p.y - ee, q.p.z - ee), q.lod);
-        q1 = cube_sample(tex, make_float3(q.p.x - ee, q.p.y - ee, q.p.z + ee), q.lod);
-        q2 = cube_sample(tex, make_float3(q.p.x - ee, q.p.y + ee, q.p.z - ee), q.lod);
-        q3 = cube_sample(tex, make_float3(q.p.x + ee, q.p.y + ee, q.p.z + ee), q.lod);
+        const float ee = (vc.voxel * q.lod_step) * ir3;
+        const CubeLevels l = cube_levels(tex, q.lod);
+        float t[4];
+        cube_taps4<kQuad>(tex, l.m, q.p, ee, t);
+        if (l.fr > 0.0f) {
+          float u[4];
+          cube_taps4<kQuad>(tex, l.m + 1u, q.p, ee, u);
+#pragma unroll
+          for (int k = 0; k < 4; k++) t[k] = lerp_(t[k], u[k], l.fr);
+        }
+        q0 = t[0], q1 = t[1], q2 = t[2], q3 = t[3];
       }
       g0 = (((q0 - q1) - q2) + q3) * renorm;
       g1 = (((-q0 - q1) + q2) + q3) * renorm;
@@ -1260,12 +1387,12 @@ __device__ __forceinline__ float3 sample_color(const DevScene &s, const ViewCons
         const float ev = q.lod_step;
         const float3 u = q.bl, org = shard_slot_org(s.sh, q.slot);
         const float e2 = r3d_exp2f(q.lod);
-        g0 = shard_fetch(s.sh, org, make_float3(u.x + ev, u.y, u.z), q.lod, e2) -
-             shard_fetch(s.sh, org, make_float3(u.x - ev, u.y, u.z), q.lod, e2);
-        g1 = shard_fetch(s.sh, org, make_float3(u.x, u.y + ev, u.z), q.lod, e2) -
-             shard_fetch(s.sh, org, make_float3(u.x, u.y - ev, u.z), q.lod, e2);
-        g2 = shard_fetch(s.sh, org, make_float3(u.x, u.y, u.z + ev), q.lod, e2) -
-             shard_fetch(s.sh, org, make_float3(u.x, u.y, u.z - ev), q.lod, e2);
+        g0 = shard_fetch<kQuad>(s.sh, org, make_float3(u.x + ev, u.y, u.z), q.lod, e2) -
+             shard_fetch<kQuad>(s.sh, org, make_float3(u.x - ev, u.y, u.z), q.lod, e2);
+        g1 = shard_fetch<kQuad>(s.sh, org, make_float3(u.x, u.y + ev, u.z), q.lod, e2) -
+             shard_fetch<kQuad>(s.sh, org, make_float3(u.x, u.y - ev, u.z), q.lod, e2);
+        g2 = shard_fetch<kQuad>(s.sh, org, make_float3(u.x, u.y, u.z + ev), q.lod, e2) -
+             shard_fetch<kQuad>(s.sh, org, make_float3(u.x, u.y, u.z - ev), q.lod, e2);
       } else if (kSection) {  // a tap moves one axis of the sample's lookup
         const float e = vc.voxel * q.lod_step;
         if (PATH == PATH_CLIP && (int)q.slot < 0) {  // as above
@@ -1314,13 +1441,19 @@ __device__ __forceinline__ float3 sample_color(const DevScene &s, const ViewCons
           }
         }
       } else {
-        float e = vc.voxel * q.lod_step;
-        g0 = cube_sample(tex, make_float3(q.p.x + e, q.p.y, q.p.z), q.lod) -
-             cube_sample(tex, make_float3(q.p.x - e, q.p.y, q.p.z), q.lod);
-        g1 = cube_sample(tex, make_float3(q.p.x, q.p.y + e, q.p.z), q.lod) -
-             cube_sample(tex, make_float3(q.p.x, q.p.y - e, q.p.z), q.lod);
-        g2 = cube_sample(tex, make_float3(q.p.x, q.p.y, q.p.z + e), q.lod) -
-             cube_sample(tex, make_float3(q.p.x, q.p.y, q.p.z - e), q.lod);
+        const float e = vc.voxel * q.lod_step;
+        const CubeLevels l = cube_levels(tex, q.lod);
+        float t[6];
+        cube_taps6<kQuad>(tex, l.m, q.p, e, t);
+        if (l.fr > 0.0f) {
+          float u[6];
+          cube_taps6<kQuad>(tex, l.m + 1u, q.p, e, u);
+#pragma unroll
+          for (int k = 0; k < 6; k++) t[k] = lerp_(t[k], u[k], l.fr);
+        }
+        g0 = t[0] - t[1];
+        g1 = t[2] - t[3];
+        g2 = t[4] - t[5];
       }
     }
     float3 gv = make_float3(g0, g1, g2);
@@ -1439,7 +1572,7 @@ template <int PATH, int MODE, bool FAST, bool COUNT, bool DEFER = false, bool OV
 __device__ __forceinline__ int ray_step(const DevScene &s, const ViewConst &vc, const float4 *tf,
                                         RayState &st, Pending &pend, const StageBox *box = nullptr) {
   constexpr bool kLod = PATH == PATH_LOD_BRICKS;
-  constexpr bool kShard = PATH == PATH_SHARD;
+  constexpr bool kShard = kShardPath<PATH>, kQuad = kQuadPath<PATH>;
   constexpr bool kSlab = PATH == PATH_SLAB;
   constexpr bool kClip = PATH == PATH_CLIP;
   constexpr bool kVslab = PATH == PATH_VSLAB;
@@ -1471,6 +1604,11 @@ __device__ __forceinline__ int ray_step(const DevScene &s, const ViewConst &vc, 
 
   float v = 0.0f;
   BrickCtx b;
+  // the occupancy byte of the skip, loaded beside the sample: the void steps
+  // that read it are most of a march, and one load behind the other was the
+  // longest wait of theirs
+  constexpr bool kOcc = !kLod && !kSlab && !kClip && !kVslab;
+  const uint32_t occ = kOcc ? occ_byte(kShard ? s.sh.atlas : s.cube, p) : 0u;
   if (kLod) {
     const int top = (int)s.br.nlev - 1;
     int desired = st.lc.desired;
@@ -1539,7 +1677,7 @@ __device__ __forceinline__ int ray_step(const DevScene &s, const ViewConst &vc, 
   } else if (kShard) {
     const DevShard &h = s.sh;
     if (h.identity) {  // atlas layout == world layout (raycast.slang:800-805)
-      v = cube_sample(h.atlas, p, lod);
+      v = cube_sample<kQuad>(h.atlas, p, lod);
     } else {
       // page entry cached until the brick changes (raycast.slang:806-822)
       const float3 vp = make_float3(sat_(p.x) * h.n, sat_(p.y) * h.n, sat_(p.z) * h.n);
@@ -1554,7 +1692,7 @@ __device__ __forceinline__ int ray_step(const DevScene &s, const ViewConst &vc, 
       }
       b = st.lc.c;
       b.bl = make_float3(vp.x - (float)(bx << 7), vp.y - (float)(by << 7), vp.z - (float)(bz << 7));
-      v = b.ok ? shard_fetch(h, shard_slot_org(h, b.slot), b.bl, lod,
+      v = b.ok ? shard_fetch<kQuad>(h, shard_slot_org(h, b.slot), b.bl, lod,
                              lod == 0.0f ? 1.0f : r3d_exp2f(lod))
                : 0.0f;
     }
@@ -1567,7 +1705,7 @@ __device__ __forceinline__ int ray_step(const DevScene &s, const ViewConst &vc, 
     b.slot = (uint32_t)cl;
     v = cl < 0 ? 0.0f : sec_sample<PATH_CLIP>(s, cl, p);
   } else {
-    v = cube_sample(s.cube, p, lod);
+    v = cube_sample<kQuad>(s.cube, p, lod);
   }
   const bool cut = v < vc.threshold;  // raycast.slang:826-827
   if (cut) v = 0.0f;
@@ -1583,21 +1721,21 @@ __device__ __forceinline__ int ray_step(const DevScene &s, const ViewConst &vc, 
   } else if (kShard) {
     if (v < vc.bgate) {
       if (s.sh.identity) {  // 8^3 occupancy only
-        if (occ_sample(s.sh.atlas, p) < vc.bgate) {
-          st.t = skip_block(st, p, vc.bs);
+        if (byte_float(occ) * kInv255 < vc.bgate) {
+          st.t = skip_block(st, p, vc.bs, vc.rbs);
           return kStepCont;
         }
       } else if (b.maxv < vc.bgate) {  // whole brick (cached page entry)
-        st.t = skip_block(st, p, 128.0f * vc.voxel);
+        st.t = skip_block(st, p, 128.0f * vc.voxel, 1.0f / (128.0f * vc.voxel));
         return kStepCont;
-      } else if (occ_sample(s.sh.atlas, p) < vc.bgate) {  // 8^3 block
-        st.t = skip_block(st, p, vc.bs);
+      } else if (byte_float(occ) * kInv255 < vc.bgate) {  // 8^3 block
+        st.t = skip_block(st, p, vc.bs, vc.rbs);
         return kStepCont;
       }
     }
   } else if (!kSlab && !kClip && !kVslab && v < vc.occ_gate &&
-             occ_sample(s.cube, p) < vc.occ_gate) {
-    st.t = skip_block(st, p, vc.bs);  // (no empty-space skip in slab mode: raycast.slang:861)
+             byte_float(occ) * kInv255 < vc.occ_gate) {
+    st.t = skip_block(st, p, vc.bs, vc.rbs);  // (no empty-space skip in slab mode: raycast.slang:861)
     return kStepCont;
   }
 
@@ -1851,7 +1989,7 @@ __device__ __forceinline__ void march_queued(const r3d_frame_params &pc, const D
     if (add) {
       if (r >= kStepShade) {
         const uint32_t e = (head + n + (uint32_t)__popc(add & below)) & 63u;
-        const bool in_slot = PATH == PATH_LOD_BRICKS || (PATH == PATH_SHARD && !s.sh.identity);
+        const bool in_slot = PATH == PATH_LOD_BRICKS || (kShardPath<PATH> && !s.sh.identity);
         const float3 at = in_slot ? pend.bl : pend.p;
         q.a[e] = make_float4(at.x, at.y, at.z, pend.tt);
         q.b[e] = make_float4(PATH == PATH_LOD_BRICKS ? pend.grad_vox : pend.lod, pend.lod_step,

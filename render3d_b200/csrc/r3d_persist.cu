@@ -20,8 +20,8 @@
 
 // Resident 128-thread blocks per SM the whole-tile kernel's registers are
 // bounded for: as the one-thread-per-ray kernels (8 for the plain LOD-brick
-// kernels, 9 for their MIP, 7 elsewhere), except the LOD-brick FULL kernel
-// (R3D_TILES_FULL_BLOCKS).
+// kernels, 9 for their MIP, kQuadBlocks on the quad paths, 7 elsewhere), except
+// the LOD-brick FULL kernel (R3D_TILES_FULL_BLOCKS).
 #ifndef R3D_TILES_FULL_BLOCKS
 #define R3D_TILES_FULL_BLOCKS 8
 #endif
@@ -30,7 +30,7 @@
                              ? (MODE == R3D_MODE_MIP     ? 9                                \
                                 : MODE == R3D_MODE_FULL ? R3D_TILES_FULL_BLOCKS            \
                                                         : 8)                               \
-                             : 7)
+                         : kQuadPath<PATH> ? kQuadBlocks<PATH>(MODE == R3D_MODE_FULL) : 7)
 
 namespace r3d {
 
@@ -407,7 +407,7 @@ static cudaError_t launch_pm(const PersistLaunch &L, const DevScene &s, cudaStre
 }
 
 #ifdef R3D_FWD_PATH
-// Compiled once per sampling path (R3D_FWD_PATH = 0..5), as the forward
+// Compiled once per sampling path (R3D_FWD_PATH = 0..7), as the forward
 // kernels are.
 template <>
 cudaError_t persist_path<R3D_FWD_PATH>(const PersistLaunch &L, const DevScene &s,
@@ -443,23 +443,27 @@ int persist_occupancy<R3D_FWD_PATH>(uint32_t mode, bool fast, uint32_t unroll) {
 }
 #else
 cudaError_t launch_persist(const PersistLaunch &L, const DevScene &s, cudaStream_t st) {
-  switch (L.path) {
+  switch (quad_path(L.path, &s, 1u)) {
     case PATH_VSLAB: return persist_path<PATH_VSLAB>(L, s, st);
     case PATH_CLIP: return persist_path<PATH_CLIP>(L, s, st);
     case PATH_SLAB: return persist_path<PATH_SLAB>(L, s, st);
     case PATH_LOD_BRICKS: return persist_path<PATH_LOD_BRICKS>(L, s, st);
     case PATH_SHARD: return persist_path<PATH_SHARD>(L, s, st);
+    case PATH_SHARD_QUAD: return persist_path<PATH_SHARD_QUAD>(L, s, st);
+    case PATH_CUBE_QUAD: return persist_path<PATH_CUBE_QUAD>(L, s, st);
     default: return persist_path<PATH_CUBE>(L, s, st);
   }
 }
 
 cudaError_t launch_tiles(const TilesLaunch &L, cudaStream_t st) {
-  switch (L.path) {
+  switch (quad_path(L.path, L.scenes, L.nscenes)) {
     case PATH_VSLAB: return tiles_path<PATH_VSLAB>(L, st);
     case PATH_CLIP: return tiles_path<PATH_CLIP>(L, st);
     case PATH_SLAB: return tiles_path<PATH_SLAB>(L, st);
     case PATH_LOD_BRICKS: return tiles_path<PATH_LOD_BRICKS>(L, st);
     case PATH_SHARD: return tiles_path<PATH_SHARD>(L, st);
+    case PATH_SHARD_QUAD: return tiles_path<PATH_SHARD_QUAD>(L, st);
+    case PATH_CUBE_QUAD: return tiles_path<PATH_CUBE_QUAD>(L, st);
     default: return tiles_path<PATH_CUBE>(L, st);
   }
 }

@@ -71,9 +71,6 @@ __global__ void k_shard_occ_raw(const uint8_t *__restrict__ atlas, uint32_t abpa
 }
 
 // Defined in r3d_ctx.cu.
-__global__ void k_downsample_clamp(const uint8_t *__restrict__ src, uint32_t sx, uint32_t sy,
-                                   uint32_t sz, uint8_t *__restrict__ dst, uint32_t dx,
-                                   uint32_t dy, uint32_t dz);
 __global__ void k_occ_dilate(const uint8_t *__restrict__ raw, uint8_t *__restrict__ dil,
                              uint32_t ox, uint32_t oy, uint32_t oz);
 
@@ -130,14 +127,23 @@ int r3d_cuda_shard_build(r3d_cuda_ctx *c, uint32_t edge, const uint8_t *voxels, 
   const size_t vbytes = (size_t)edge * edge * edge;
 
   R3D_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+  // the atlas, its occupancy (and the raw grid) and quad words in one
+  // allocation, kept when about this size (the words alone when the whole does
+  // not fit), and the builder's tables with the page table in another
   uint8_t *buf = nullptr, *vtmp = nullptr;
-  uint32_t *dslot = nullptr, *dbrick = nullptr, *dmax = nullptr, *dpage = nullptr;
-  const bool dev_in = is_device_ptr(voxels) && ((uintptr_t)voxels & 15u) == 0u;
-  cudaError_t e = cudaMalloc(&buf, total + onb);
-  if (e == cudaSuccess) e = cudaMalloc(&dslot, sizeof(uint32_t) * nb);
-  if (e == cudaSuccess) e = cudaMalloc(&dbrick, sizeof(uint32_t) * ns);
-  if (e == cudaSuccess) e = cudaMalloc(&dmax, sizeof(uint32_t) * nb);
-  if (e == cudaSuccess) e = cudaMalloc(&dpage, sizeof(uint32_t) * nb);
+  uint32_t *dpage = nullptr;
+  const bool dev_in = readable_in_place(c, voxels) && ((uintptr_t)voxels & 15u) == 0u;
+  const size_t base = (total + onb + 255) & ~(size_t)255, qbytes = cube_quad_bytes(h.atlas);
+  const bool kept = keeps(c->shard_buf, c->shard_cap, base + qbytes);
+  bool whole = true;
+  cudaError_t e = kept ? cudaDeviceSynchronize() : cudaMalloc(&buf, base + qbytes);
+  if (e == cudaErrorMemoryAllocation && qbytes) {
+    cudaGetLastError();
+    whole = false;
+    e = cudaMalloc(&buf, base);
+  }
+  if (e == cudaSuccess) e = cudaMalloc(&dpage, sizeof(uint32_t) * (3u * (size_t)nb + ns));
+  uint32_t *const dslot = dpage + nb, *const dmax = dslot + nb, *const dbrick = dmax + nb;
   if (e == cudaSuccess && !dev_in) e = cudaMalloc(&vtmp, vbytes);
   const uint8_t *vol = dev_in ? voxels : vtmp;
   if (e == cudaSuccess && !dev_in)
@@ -150,6 +156,10 @@ int r3d_cuda_shard_build(r3d_cuda_ctx *c, uint32_t edge, const uint8_t *voxels, 
                         c->stream);
   std::vector<uint32_t> maxv(nb);
   if (e == cudaSuccess) {
+    if (kept) {
+      buf = c->shard_buf;
+      c->have_shard = false;
+    }
     k_shard_place<<<shard_grid((size_t)a * a * a / 16u), 256, 0, c->stream>>>(vol, edge, bpa,
                                                                              dbrick, abpa, buf);
     // the display filter on the placed slots, before the mips and the
@@ -162,11 +172,8 @@ int r3d_cuda_shard_build(r3d_cuda_ctx *c, uint32_t edge, const uint8_t *voxels, 
       if (frc != R3D_OK) {
         cudaStreamSynchronize(c->stream);
         cudaFree(vtmp);
-        cudaFree(dslot);
-        cudaFree(dbrick);
-        cudaFree(dmax);
         cudaFree(dpage);
-        cudaFree(buf);
+        if (!kept) cudaFree(buf);
         return frc;
       }
     }
@@ -177,8 +184,7 @@ int r3d_cuda_shard_build(r3d_cuda_ctx *c, uint32_t edge, const uint8_t *voxels, 
                             c->stream);
     for (uint32_t m = 1; m < 4u; m++) {
       const uint32_t s = a >> (m - 1), d = a >> m;
-      k_downsample_clamp<<<shard_grid((size_t)d * d * d), 256, 0, c->stream>>>(
-          buf + off[m - 1], s, s, s, buf + off[m], d, d, d);
+      if (e == cudaSuccess) e = launch_mip(buf + off[m - 1], s, s, s, buf + off[m], d, d, d, c->stream);
     }
     k_shard_occ_raw<<<shard_grid(onb), 256, 0, c->stream>>>(buf, abpa, dslot, bpa, buf + total);
     k_occ_dilate<<<shard_grid(onb), 256, 0, c->stream>>>(buf + total, buf + off[4], od, od, od);
@@ -194,11 +200,8 @@ int r3d_cuda_shard_build(r3d_cuda_ctx *c, uint32_t edge, const uint8_t *voxels, 
   if (e == cudaSuccess)
     e = copy_sync(c->stream, dpage, page.data(), sizeof(uint32_t) * nb);
   cudaFree(vtmp);
-  cudaFree(dslot);
-  cudaFree(dbrick);
-  cudaFree(dmax);
   if (e != cudaSuccess) {
-    cudaFree(buf);
+    if (!kept) cudaFree(buf);
     cudaFree(dpage);
     return cuda_fail(c, e, "shard_build");
   }
@@ -210,10 +213,22 @@ int r3d_cuda_shard_build(r3d_cuda_ctx *c, uint32_t edge, const uint8_t *voxels, 
   h.n = (float)edge;
   h.inv_adim = 1.0f / ((float)abpa * 128.0f);  // raycast.slang:758
   h.identity = identity ? 1u : 0u;
-  cudaFree(c->shard_buf);
+  if (!kept) {
+    cudaFree(c->shard_buf);
+    c->shard_buf = buf;
+    c->shard_cap = whole ? base + qbytes : base;
+  }
   cudaFree(c->shard_page);
-  c->shard_buf = buf;
   c->shard_page = dpage;
+  c->have_shard = false;
+  cudaFree(c->shard_quad);
+  c->shard_quad = nullptr;
+  uint32_t *words = whole && qbytes ? (uint32_t *)(buf + base) : nullptr;
+  if (!whole && cudaMalloc(&c->shard_quad, qbytes) == cudaSuccess) words = c->shard_quad;
+  if (!whole) cudaGetLastError();
+  e = build_cube_quads(h.atlas, words, c->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  if (e != cudaSuccess) return cuda_fail(c, e, "shard_build: quad words");
   c->sh = h;
   c->have_shard = true;
   return R3D_OK;

@@ -1,4 +1,4 @@
-"""r3d_div_by against IEEE division, compiled from the header as the kernels'
+"""r3d_div_by and r3d_div_rcp against IEEE division, compiled from the header as the kernels'
 host twin: every divisor up to 8200 (tile and ring sizes and far beyond), and
 powers of two and their neighbours up to the stated bound, with random
 dividends, whole ones, and the ones nearest to a rounding boundary (b times a
@@ -31,6 +31,23 @@ static long divisor(uint32_t b, int n) {
   }
   return bad + check(0.0f, b);
 }
+/* any divisor: dividends near a rounding boundary of the quotient too */
+long run_rcp(void) {
+  long bad = 0;
+  for (int i = 0; i < 4000000; i++) {
+    uint32_t r = rnd(), q = rnd();
+    float b = r3d_u2f((r & 0x807fffffu) | ((100u + rnd() % 40u) << 23));
+    if (i % 4 == 0) b = r3d_u2f((r & 0x80000007u) | ((100u + rnd() % 40u) << 23) | (i % 8 ? 0x7ffff8u : 0u));
+    float rb = 1.0f / b, a = r3d_u2f((q & 0x807fffffu) | ((100u + rnd() % 40u) << 23));
+    if (i & 1) {
+      double mid = ((double)(q & 0xffffffu) * 2.0 + 1.0 + 0x1000000) * (double)b;
+      a = (float)(mid * (i & 2 ? 0x1p-30 : 0x1p-8));
+    }
+    for (int k = 0; k < 3; k++, a = nextafterf(a, INFINITY))
+      bad += r3d_f2u(a / b) != r3d_f2u(r3d_div_rcp(a, b, rb));
+  }
+  return bad + (r3d_f2u(0.0f / 3.0f) != r3d_f2u(r3d_div_rcp(0.0f, 3.0f, 1.0f / 3.0f)));
+}
 long run(void) {
   long bad = 0;
   for (uint32_t b = 1; b <= 8200u; b++) bad += divisor(b, 400);
@@ -49,5 +66,6 @@ def test_div_by_is_ieee_division(tmp_path):
                     "-shared", "-fPIC", "-I" + os.path.join(ROOT, "include"), str(c), "-o", str(so),
                     "-lm"], check=True)
     lib = ctypes.CDLL(str(so))
-    lib.run.restype = ctypes.c_long
-    assert lib.run() == 0
+    for fn in (lib.run, lib.run_rcp):
+        fn.restype = ctypes.c_long
+        assert fn() == 0
