@@ -141,6 +141,42 @@ R3D_FM_HD float r3d_exp2f(float x) {
   return a * r3d_u2f((uint32_t)(n2 + 127) << 23);
 }
 
+/* r3d_log2f(x) for x >= 1, without its special cases (+inf gives 128): the
+ * split at sqrt(2) is one subtraction on the bits, whose borrow is the
+ * exponent's carry.  The footprint ratio of a sample is such an x. */
+R3D_FM_HD float r3d_log2_ge1f(float x) {
+  const uint32_t k = 0x3f3504f4u; /* half the first float above 1.41421356f */
+  const uint32_t b = r3d_f2u(x) - k;
+  const uint32_t e = b >> 23;
+  const float m = r3d_u2f((b & 0x007fffffu) + k);
+#if defined(__CUDA_ARCH__)
+  const float s = r3d_atanh_arg(m);
+#else
+  const float s = (m - 1.0f) / (m + 1.0f);
+#endif
+  const float s2 = s * s;
+  float p = fmaf(s2, 0.111111111f, 0.142857143f);
+  p = fmaf(s2, p, 0.2f);
+  p = fmaf(s2, p, 0.333333333f);
+  p = fmaf(s2, p, 1.0f);
+  return (r3d_u2f(0x4B400000u + e) - 12582912.0f) + (s * 2.88539008f) * p;
+}
+
+/* r3d_exp2f(x) for 0 <= x <= 126, without its special cases: the result is
+ * normal, so the scale is an addition to the exponent field. */
+R3D_FM_HD float r3d_exp2_posf(float x) {
+  const float big = x + 12582912.0f;
+  const float f = x - (big - 12582912.0f);
+  float p = fmaf(f, 1.52527338e-05f, 1.54035304e-04f);
+  p = fmaf(f, p, 1.33335581e-03f);
+  p = fmaf(f, p, 9.61812911e-03f);
+  p = fmaf(f, p, 5.55041087e-02f);
+  p = fmaf(f, p, 2.40226507e-01f);
+  p = fmaf(f, p, 6.93147181e-01f);
+  p = fmaf(f, p, 1.0f);
+  return r3d_u2f(r3d_f2u(p) + (r3d_f2u(big) << 23));
+}
+
 /* x^y for x >= 0 (the only use here): 0^y = 0 for y > 0, x^0 = 1. */
 R3D_FM_HD float r3d_powf(float x, float y) {
   if (y == 0.0f || x == 1.0f) return 1.0f;

@@ -511,7 +511,7 @@ __device__ __forceinline__ BrickCtx lod_locate_ex(const DevScene &s, float3 p, f
     c.slot = slot;
     c.bl = make_float3(lv[0] - (float)(bc[0] << 7), lv[1] - (float)(bc[1] << 7),
                        lv[2] - (float)(bc[2] << 7));
-    c.grad_vox = r3d_exp2f(lod) * inv;
+    c.grad_vox = r3d_exp2_posf(lod) * inv;
     c.world_brick = (128.0f * (float)b.scale[li]) / b.md;
     inv_out = inv;
     bco[0] = bc[0];
@@ -533,27 +533,25 @@ __device__ __forceinline__ BrickCtx lod_locate_ex(const DevScene &s, float3 p, f
 // p are the cached ones.  The test runs on bl = lv - lo: rounding keeps the
 // sign of a difference, and for lo <= lv < lo + 128 the difference is exact
 // (lo = 0, or lv <= 2 lo), so bl >= 0 && bl < 128 decides exactly what
-// lo <= lv < lo + 128 does, and an empty cache (lo = +inf) never hits.
+// lo <= lv < lo + 128 does, and an empty cache (lo = +inf) never hits.  On
+// the bits as unsigned numbers that is one comparison with 128.0f, for the
+// largest of the three: a negative difference, -0 and NaN are above it.  So
+// the clamp of lv at 0 is left to the walk too, which every miss takes and
+// which finds the same brick (with six float compares and both clamps the
+// 1080p orbit took 407 us FULL, 803 MIP, 489 HEATMAP; now 397, 747, 449).
 __device__ __forceinline__ bool lod_cache_hit(const DevScene &s, float3 p, int desired,
                                               const LodCache &lc, BrickCtx &out) {
   const DevBricks &b = s.br;
-  if (lc.desired == desired) {
-    float bl[3];
-    bool same = true;
-    float pv[3] = {p.x, p.y, p.z};
+  float bl[3];
+  const float pv[3] = {p.x, p.y, p.z};
 #pragma unroll
-    for (int a = 0; a < 3; a++) {
-      float base_v = clamp_(pv[a] * b.md, 0.0f, b.bs_hi[a]);
-      bl[a] = base_v * lc.inv_scale - lc.lo[a];
-      same = same && bl[a] >= 0.0f && bl[a] < 128.0f;
-    }
-    if (same) {
-      out = lc.c;
-      out.bl = make_float3(bl[0], bl[1], bl[2]);
-      return true;
-    }
-  }
-  return false;
+  for (int a = 0; a < 3; a++) bl[a] = fminf(pv[a] * b.md, b.bs_hi[a]) * lc.inv_scale - lc.lo[a];
+  const uint32_t most =
+      max(max(__float_as_uint(bl[0]), __float_as_uint(bl[1])), __float_as_uint(bl[2]));
+  if (most >= 0x43000000u || lc.desired != desired) return false;  // 128.0f
+  out = lc.c;
+  out.bl = make_float3(bl[0], bl[1], bl[2]);
+  return true;
 }
 
 // Slot-local texel coordinates of bricks_fetch (clamped, minus 0.5) and
@@ -1591,12 +1589,15 @@ __device__ __forceinline__ int ray_step(const DevScene &s, const ViewConst &vc, 
     } else {
       // a footprint under a voxel is clamped to y = 1, whose logarithm is 0
       const float y = lod_y(vc, t);
-      lod = clamp_((!kLod && y == 1.0f ? 0.0f : r3d_log2f(y)) + vc.lod_bias, 0.0f, vc.max_lod);
+      lod = clamp_((!kLod && y == 1.0f ? 0.0f : r3d_log2_ge1f(y)) + vc.lod_bias, 0.0f, vc.max_lod);
     }
   }
-  float lod_step =
-      !lod_known || st.span_dom ? st.span_step
-                                : fmaxf(lod == 0.0f ? 1.0f : r3d_exp2f(lod), st.span_step);
+  float lod_step = st.span_step;
+  if (kLod) {  // 0 <= lod < nlev
+    if (lod_known) lod_step = fmaxf(r3d_exp2_posf(lod), st.span_step);
+  } else if (!st.span_dom) {
+    lod_step = fmaxf(lod == 0.0f ? 1.0f : r3d_exp2f(lod), st.span_step);
+  }
   if (kSlab || kClip || kVslab) lod_step = fminf(lod_step, st.slab_cap);
   const float3 dir = st.dir;
   const float3 p =
@@ -1613,11 +1614,11 @@ __device__ __forceinline__ int ray_step(const DevScene &s, const ViewConst &vc, 
     const int top = (int)s.br.nlev - 1;
     int desired = st.lc.desired;
     if (lod_known) {
-      desired = (int)clamp_(floorf(lod), 0.0f, (float)top);
+      desired = min((int)(__float_as_uint(__fadd_rz(lod, 8388608.0f)) & 0x7fffffu), top);
       if (desired != st.lc.desired) lod_range(st, vc, desired, top);
     }
     if (!lod_cache_hit(s, p, desired, st.lc, b)) {  // walk the page table
-      if (!lod_known) lod = clamp_(r3d_log2f(lod_y(vc, t)) + vc.lod_bias, 0.0f, vc.max_lod);
+      if (!lod_known) lod = clamp_(r3d_log2_ge1f(lod_y(vc, t)) + vc.lod_bias, 0.0f, vc.max_lod);
       if (COUNT) st.n_walk++;
       b = lod_locate_ex(s, p, lod, st.lc, desired);
     }
