@@ -144,7 +144,6 @@ int r3d_cuda_create(int device, r3d_cuda_ctx **out) {
       r3d_cuda_destroy(c);
       return R3D_E_CUDA;
     }
-  if (cudaMalloc(&c->cube_small, kSmallCube) != cudaSuccess) cudaGetLastError();
   // default transfer function: grey ramp with alpha = value
   // (src/vk/vkbackend.c:1100-1114)
   uint8_t ramp[256][4];
@@ -162,7 +161,6 @@ void r3d_cuda_destroy(r3d_cuda_ctx *c) {
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
   cudaFree(c->cube_buf);
-  cudaFree(c->cube_small);
   cudaFree(c->cube_quad);
   cudaFree(c->shard_quad);
   cudaFree(c->page);
@@ -247,8 +245,7 @@ int r3d_cuda_upload_volume(r3d_cuda_ctx *c, const r3d_volume_desc *d, const uint
   // kept when about this size as the brick cache's are; the words stand alone
   // when the whole does not fit beside the volume it replaces
   const size_t base = (total + onb + 255) & ~(size_t)255, qbytes = cube_quad_bytes(cube);
-  const bool tiny = c->cube_small && base + qbytes <= kSmallCube;
-  const bool kept = tiny || keeps(c->cube_buf, c->cube_cap, base + qbytes);
+  const bool kept = keeps(c->cube_buf, c->cube_cap, base + qbytes);
   bool whole = true;
   cudaError_t e = kept ? cudaDeviceSynchronize() : cudaMalloc(&buf, base + qbytes);
   if (e == cudaErrorMemoryAllocation && qbytes) {
@@ -258,7 +255,7 @@ int r3d_cuda_upload_volume(r3d_cuda_ctx *c, const r3d_volume_desc *d, const uint
   }
   if (e != cudaSuccess) return cuda_fail(c, e, "upload_volume: cudaMalloc");
   if (kept) {
-    buf = tiny ? c->cube_small : c->cube_buf;
+    buf = c->cube_buf;
     c->have_cube = false;
   }
   raw = buf + total;
@@ -279,10 +276,10 @@ int r3d_cuda_upload_volume(r3d_cuda_ctx *c, const r3d_volume_desc *d, const uint
     if (!kept) cudaFree(buf);
     return cuda_fail(c, e, "upload_volume");
   }
-  if (tiny || !kept) {
+  if (!kept) {
     cudaFree(c->cube_buf);
-    c->cube_buf = tiny ? nullptr : buf;
-    c->cube_cap = tiny ? 0 : whole ? base + qbytes : base;
+    c->cube_buf = buf;
+    c->cube_cap = whole ? base + qbytes : base;
   }
   c->have_cube = false;
   c->cube.quad = nullptr;

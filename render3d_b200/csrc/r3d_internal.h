@@ -17,7 +17,6 @@ struct r3d_cuda_ctx {
 
   // cube volume: all mip levels in one allocation, then the occupancy grid
   uint8_t *cube_buf = nullptr;
-  uint8_t *cube_small = nullptr;  // kSmallCube bytes, for the cubes that fit
   size_t cube_bytes = 0, cube_cap = 0;
   uint32_t *cube_quad = nullptr;  // the cube's quad words when not in cube_buf
   bool have_cube = false;
@@ -197,10 +196,6 @@ namespace r3d {
 inline bool keeps(const void *p, size_t cap, size_t need) {
   return p && cap >= need && need > cap / 2;
 }
-// Cubes of up to this many bytes with their tables lie in a buffer that the
-// context is created with: a cudaMalloc beyond the driver's current 2 MB takes
-// 0.4 ms, four times the upload of a 96^3 volume (0.12 ms).
-constexpr size_t kSmallCube = (size_t)8 << 20;
 
 int fail(r3d_cuda_ctx *c, int code, const char *fmt, ...);
 int cuda_fail(r3d_cuda_ctx *c, cudaError_t e, const char *what);
