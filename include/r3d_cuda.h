@@ -449,9 +449,7 @@ int r3d_cuda_raycast_fwd_noalloc(r3d_cuda_ctx *ctx, const r3d_frame_params *view
  * limit).  shade_group (FULL mode, one-thread-per-ray launches): n > 0
  * leaves samples that need gradient shading in a queue of the warp until n
  * of them wait, and shades them together, one per lane (1: as soon as a step
- * of the warp leaves any); 0 picks the sampling path's default: 32 on the
- * cube, shard, tiled-slab, clipmap and virtual-slab paths, and shading where
- * the ray meets the sample for LOD bricks.  Results are identical under every
+ * of the warp leaves any); 0 is 32.  Results are identical under every
  * schedule. */
 typedef struct r3d_cuda_schedule {
   uint32_t persistent;

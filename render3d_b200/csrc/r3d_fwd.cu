@@ -9,10 +9,10 @@
 
 // Minimum resident 128-thread blocks per SM the register allocator targets
 // (0: no target).  The plain LOD-brick kernels (no overlay atlases, counters
-// or parked shading, not the step heatmap) get one block more, MIP two, all
-// without spills: 1080p FULL runs 2 % faster at 64 registers and MIP 5 %
-// at 56, while the overlay and shard kernels lose 14 % and 4 % and the
-// heatmap 3 % at 8 blocks, and FULL spills at 9.  The quad paths: kQuadBlocks.
+// or shading queue, not the step heatmap) get one block more, MIP two, all
+// without spills: MIP runs 5 % faster at 56 registers, while the overlay and
+// shard kernels lose 14 % and 4 % and the heatmap 3 % at 8 blocks, and FULL,
+// with its queue, spills there.  The quad paths: kQuadBlocks.
 #ifndef R3D_FWD_MIN_BLOCKS
 #define R3D_FWD_MIN_BLOCKS 7
 #endif
@@ -160,9 +160,7 @@ static cudaError_t launch_t(const r3d_frame_params &pc, const DevScene &s, const
   if (row0 >= row1) return cudaSuccess;
   dim3 grid((gw + kBlockW - 1u) / kBlockW, (row1 - row0 + kBlockH - 1u) / kBlockH);
   const uint32_t threads = kFwdWarps * 32u;
-  // FULL views with and without the queue: LOD bricks (by the schedule); the
-  // other paths' FULL views always queue
-  constexpr bool kQueue = MODE == R3D_MODE_FULL, kDirect = !kQueue || !kShadeQueued<PATH, MODE, false>;
+  constexpr bool kQueue = kShadeQueued<PATH, MODE, false>;
   // overlay atlases: LOD bricks in the compositing and MIP modes
   constexpr bool kOvl = PATH == PATH_LOD_BRICKS &&
                         (MODE == R3D_MODE_FULL || MODE == R3D_MODE_FLAT || MODE == R3D_MODE_MIP);
@@ -178,18 +176,14 @@ static cudaError_t launch_t(const r3d_frame_params &pc, const DevScene &s, const
     }
   }
   if constexpr (kQueue) {
-    if (shade || !kDirect) {
-      if (!shade) shade = 32u;
-      if (counters)
-        k_raycast<PATH, MODE, FAST, true, true><<<grid, threads, 0, stream>>>(
-            pc, s, lut, (uchar4 *)img, out_w, steps, mip, total, counters, shade, row0);
-      else
-        k_raycast<PATH, MODE, FAST, false, true><<<grid, threads, 0, stream>>>(
-            pc, s, lut, (uchar4 *)img, out_w, steps, mip, total, nullptr, shade, row0);
-      return cudaGetLastError();
-    }
-  }
-  if constexpr (kDirect) {
+    if (!shade) shade = 32u;
+    if (counters)
+      k_raycast<PATH, MODE, FAST, true, true><<<grid, threads, 0, stream>>>(
+          pc, s, lut, (uchar4 *)img, out_w, steps, mip, total, counters, shade, row0);
+    else
+      k_raycast<PATH, MODE, FAST, false, true><<<grid, threads, 0, stream>>>(
+          pc, s, lut, (uchar4 *)img, out_w, steps, mip, total, nullptr, shade, row0);
+  } else {
     if (counters)
       k_raycast<PATH, MODE, FAST, true, false><<<grid, threads, 0, stream>>>(
           pc, s, lut, (uchar4 *)img, out_w, steps, mip, total, counters, 0u, row0);
@@ -262,7 +256,7 @@ cudaError_t launch_view(const r3d_cuda_ctx *c, const r3d_frame_params &pc, uint8
   s.el = elide_counts(pc, s.tf_zero_t);
   const bool fast = c->quality == R3D_QUALITY_FAST;
   const int path = quad_path(path_of_view(pc), &s, 1u);
-  const uint32_t shade = c->sched.shade_group;  // 0: the path's default (kShadeQueued)
+  const uint32_t shade = c->sched.shade_group;  // 0: 32
 #define R3D_PATH_CASE(P)                                                                   \
   case P:                                                                                  \
     return launch_path<P>(pc, s, fast, c->lut, img, out_w, steps, mip_index, total, counters, \

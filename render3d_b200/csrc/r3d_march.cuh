@@ -1953,16 +1953,20 @@ __device__ __forceinline__ void shade_batch(const DevScene &s, const ViewConst &
   shade_fold(q.a, q.own, head, n, ray, st.acc_r, st.acc_g, st.acc_b);
 }
 
-// Whether a kernel's FULL views shade through the queue when the schedule
-// does not say (shade_group 0).  Measured on whole frames, queue against
-// shading in place (sections: against parking 16 lanes' samples): tiled slab
-// 2.74 -> 1.79 ms (3.8 shaded samples a pixel), virtual slab 2.13 -> 1.35,
-// 512^3 shard 1.84 -> 1.74, 256^3 cube 0.58 -> 0.57, a thumbnail 0.23 -> 0.17;
-// LOD bricks lose (1080p frame 0.507 -> 0.540, four panes 0.60 -> 0.67): a
-// tap there is two loads in the cached brick, and the votes of every step
-// cost more than the idle lanes.
-template <int PATH, int MODE, bool OVL>
-constexpr bool kShadeQueued = MODE == R3D_MODE_FULL && !OVL && PATH != PATH_LOD_BRICKS;
+// Whether a kernel's views shade through the queue.  Measured on whole frames,
+// queue against shading in place (sections: against parking 16 lanes'
+// samples): tiled slab 2.74 -> 1.79 ms (3.8 shaded samples a pixel), virtual
+// slab 2.13 -> 1.35, 512^3 shard 1.84 -> 1.74, 256^3 cube 0.58 -> 0.57, a
+// thumbnail 0.23 -> 0.17; LOD bricks in the grid kernel, where the queue fits
+// 72 registers and 7 blocks, 0.385 -> 0.371 (1080p orbit; with 8 blocks it
+// spills, 0.402; two or four steps between the votes 0.389 and 0.405).
+// LOD bricks in the whole-tile kernel spill with it: four panes alone 0.571 to
+// 0.660 ms in place against 0.605, three such calls at once 0.46 to 0.52 a call
+// against 0.53 to 0.54.  A tap there is two loads in the cached brick, and one
+// launch over many views has no idle SMs to fill, so it stays in place.
+// Overlay views shade in place: their samples carry the registration scan's.
+template <int PATH, int MODE, bool OVL, bool TILES = false>
+constexpr bool kShadeQueued = MODE == R3D_MODE_FULL && !OVL && !(TILES && PATH == PATH_LOD_BRICKS);
 
 // march() for every lane of a warp (all 32 lanes call it; `inside` says
 // whether the lane has a ray) with the shading queue: `group` waiting samples

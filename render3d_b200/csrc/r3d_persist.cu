@@ -245,7 +245,7 @@ __global__ void R3D_TILES_BOUNDS k_raycast_tiles(
     uint32_t *__restrict__ steps_out, uint32_t *__restrict__ mip_out,
     unsigned long long *__restrict__ total, unsigned long long *__restrict__ counters) {
   __shared__ float4 tf[NS][256];
-  __shared__ ShadeQueue sq[kShadeQueued<PATH, MODE, false> ? 4 : 1];
+  __shared__ ShadeQueue sq[kShadeQueued<PATH, MODE, false, true> ? 4 : 1];
   for (uint32_t k = 0; k < (NS > 1 ? sc.n : 1u); k++)
     for (uint32_t i = threadIdx.x; i < 256u; i += blockDim.x) {
       const uchar4 u = sc.lut[k][i];
@@ -273,7 +273,7 @@ __global__ void R3D_TILES_BOUNDS k_raycast_tiles(
       const bool inside = tx < v.grid_w && ty < v.grid_h;
       const uint32_t px = half ? tx * 2u : tx, py = half ? ty * 2u : ty;
       const ViewConst vc = view_const<PATH>(v.pc, s, v.el);
-      if constexpr (kShadeQueued<PATH, MODE, false>)
+      if constexpr (kShadeQueued<PATH, MODE, false, true>)
         march_queued<PATH, MODE, FAST, COUNT>(v.pc, s, vc, tf[si], px, py, inside, r,
                                               sq[threadIdx.x >> 5], 32u);
       else
