@@ -208,10 +208,15 @@ cudaError_t launch_slot_tables(const uint8_t *pool, const uint32_t *slot, uint32
   f.nlev = 0u;
   f.brick = nullptr;
   f.slot = slot;
+  // a pool handed over by a caller may start at any byte
+  const bool vec = ((uintptr_t)pool & 3u) == 0u;
   for (uint32_t j0 = 0; j0 < njobs; j0 += 65535u) {
     f.job0 = j0;
     const dim3 grid(16u, njobs - j0 < 65535u ? njobs - j0 : 65535u);
-    k_slot_fill<0, true><<<grid, 256, 0, st>>>(f, pool, nullptr, quad, bmax);
+    if (vec)
+      k_slot_fill<0, true><<<grid, 256, 0, st>>>(f, pool, nullptr, quad, bmax);
+    else
+      k_slot_fill<0, false><<<grid, 256, 0, st>>>(f, pool, nullptr, quad, bmax);
   }
   return cudaGetLastError();
 }
