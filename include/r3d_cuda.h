@@ -567,7 +567,11 @@ typedef struct r3d_cuda_grads {
 
 /* Renders nviews (1..64) views (explicit viewports, cube path, optionally
  * orthographic) into rgb_out: per view, viewport[0]*viewport[1]*3 floats,
- * views back to back.  total_steps (nullable) += march iterations. */
+ * views back to back.  total_steps (nullable) += march iterations.
+ * Differentiable calls of one context may overlap on several streams as long
+ * as they read the same density (contents too: the context keeps one packed
+ * copy of it), one tape is written or read at a time, and at most one of them
+ * is a deterministic backward (its accumulators are the context's). */
 int r3d_cuda_diff_forward(r3d_cuda_ctx *ctx, const r3d_cuda_diff_scene *scene,
                           const r3d_frame_params *views, uint32_t nviews, float *rgb_out,
                           unsigned long long *total_steps, void *stream);

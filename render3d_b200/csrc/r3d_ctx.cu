@@ -128,6 +128,9 @@ int r3d_cuda_create(int device, r3d_cuda_ctx **out) {
       cudaMalloc(&c->ring_dev, sizeof(DevView) * kMaxBatchViews * r3d_cuda_ctx::kRing) !=
           cudaSuccess ||
       cudaMalloc(&c->ring_queue, sizeof(uint32_t) * 2 * kMaxBatchViews * r3d_cuda_ctx::kRing) !=
+          cudaSuccess ||
+      cudaMalloc(&c->diff_words, sizeof(uint32_t) * 2 * (r3d_cuda_ctx::kRing +
+                                                         r3d_cuda_ctx::kCapturedCalls)) !=
           cudaSuccess) {
     cudaGetLastError();
     r3d_cuda_destroy(c);
@@ -140,7 +143,8 @@ int r3d_cuda_create(int device, r3d_cuda_ctx **out) {
     return R3D_E_CUDA;
   }
   for (int k = 0; k < r3d_cuda_ctx::kRing; k++)
-    if (cudaEventCreateWithFlags(&c->ring_ev[k], cudaEventDisableTiming) != cudaSuccess) {
+    if (cudaEventCreateWithFlags(&c->ring_ev[k], cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ring_march_ev[k], cudaEventDisableTiming) != cudaSuccess) {
       r3d_cuda_destroy(c);
       return R3D_E_CUDA;
     }
@@ -190,11 +194,14 @@ void r3d_cuda_destroy(r3d_cuda_ctx *c) {
   cudaFree(c->tape_n);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
-  for (int k = 0; k < r3d_cuda_ctx::kRing; k++)
+  for (int k = 0; k < r3d_cuda_ctx::kRing; k++) {
     if (c->ring_ev[k]) cudaEventDestroy(c->ring_ev[k]);
+    if (c->ring_march_ev[k]) cudaEventDestroy(c->ring_march_ev[k]);
+  }
   cudaFreeHost(c->ring_host);
   cudaFree(c->ring_dev);
   cudaFree(c->ring_queue);
+  cudaFree(c->diff_words);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
 }

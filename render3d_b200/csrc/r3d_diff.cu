@@ -53,7 +53,9 @@ struct DiffGrid {
   // of its z plane, x1 = min(x + 1, nx - 1) and y1 likewise, so that a
   // trilinear sample reads two float4 instead of eight floats
   const float4 *quad;
-  uint32_t *zc;  // [0]: the TF's first texel with alpha not 0 (256: none), [1]: the next ray tile
+  // the call's own words (call_words): [0] the TF's first texel with alpha not
+  // 0 (256: none), [1] the next ray tile
+  uint32_t *zc;
   uint32_t n[3];
   uint32_t nmax;
   uint32_t wide;  // an axis of more than 2^23 voxels (floor_frac's range)
@@ -238,8 +240,8 @@ __global__ void k_diff_quads(const float *__restrict__ d, uint32_t nx, uint32_t 
   }
 }
 
-// DiffGrid::zc from the TF, and the tile counter of the call's march kernel
-// (the word after it) back at 0 (one block).
+// The call's words (DiffGrid::zc): the TF's first texel with alpha, and the
+// tile counter at 0 (one block).
 __global__ void k_diff_tf_clear(const float *__restrict__ lut, uint32_t *__restrict__ zc) {
   __shared__ uint32_t z;
   if (threadIdx.x == 0) z = 256u;
@@ -679,12 +681,41 @@ __global__ void k_fix_to_float(const unsigned long long *__restrict__ q, float *
 
 using namespace r3d;
 
-// Validates the grid and views, uploads the view table; returns the grid
-// descriptor and total output floats.
+// A call's words (DiffGrid::zc).  Calls of one context may overlap on several
+// streams, and each drains its own tile counter, so the words go with the view
+// table's ring slot: the call that takes a slot again waits, on its stream, for
+// the march of the one that had it.  A call that is being captured can not
+// wait for work outside its graph, and its graph may run at any later time:
+// it takes words that only captured calls use, others for each call until
+// kCapturedCalls have been captured.
+static int call_words(r3d_cuda_ctx *c, int slot, DiffGrid &g, bool &captured, cudaStream_t st) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  R3D_CUDA_TRY(c, cudaStreamIsCapturing(st, &cs));
+  captured = cs != cudaStreamCaptureStatusNone;
+  if (!captured) {
+    g.zc = c->diff_words + 2 * slot;
+    if (c->ring_marched[slot]) R3D_CUDA_TRY(c, cudaStreamWaitEvent(st, c->ring_march_ev[slot], 0));
+  } else {
+    g.zc = c->diff_words + 2 * (r3d_cuda_ctx::kRing + c->captured_next);
+    c->captured_next = (c->captured_next + 1u) % r3d_cuda_ctx::kCapturedCalls;
+  }
+  return R3D_OK;
+}
+
+// After the march: the slot may be taken again.
+static int call_marched(r3d_cuda_ctx *c, int slot, bool captured, cudaStream_t st) {
+  if (captured) return R3D_OK;
+  R3D_CUDA_TRY(c, cudaEventRecord(c->ring_march_ev[slot], st));
+  c->ring_marched[slot] = true;
+  return R3D_OK;
+}
+
+// Validates the grid and views, takes the call's words and uploads the view
+// table; returns the grid descriptor, total output floats and ring slot.
 static int diff_prepare(r3d_cuda_ctx *c, const r3d_cuda_diff_scene *sc,
                         const r3d_frame_params *views, uint32_t nviews, DiffGrid &g,
-                        DiffView *&dviews, uint32_t &ntiles, size_t &nfloats,
-                        cudaStream_t st) {
+                        DiffView *&dviews, uint32_t &ntiles, size_t &nfloats, int &slot,
+                        bool &captured, cudaStream_t st) {
   if (!sc || !sc->density || !sc->lut || !sc->nx || !sc->ny || !sc->nz || !views || !nviews ||
       nviews > kMaxBatchViews)
     return fail(c, R3D_E_INVALID, "diff: bad arguments");
@@ -723,6 +754,9 @@ static int diff_prepare(r3d_cuda_ctx *c, const r3d_cuda_diff_scene *sc,
     tiles += (uint64_t)((p.viewport[0] + 7u) / 8u) * ((p.viewport[1] + 3u) / 4u);
   }
   ntiles = (uint32_t)tiles;  // at most 64 views of 2048 x 4096 tiles: 2^29
+  slot = k;
+  const int rc = call_words(c, slot, g, captured, st);
+  if (rc != R3D_OK) return rc;
   R3D_CUDA_TRY(c, cudaMemcpyAsync(dviews, hv, sizeof(DiffView) * nviews, cudaMemcpyHostToDevice,
                                   st));
   R3D_CUDA_TRY(c, cudaEventRecord(c->ring_ev[k], st));
@@ -735,7 +769,7 @@ static int diff_prepare(r3d_cuda_ctx *c, const r3d_cuda_diff_scene *sc,
 static int diff_quads(r3d_cuda_ctx *c, const r3d_cuda_diff_scene *sc, DiffGrid &g, bool reuse,
                       cudaStream_t st) {
   const size_t nvox = (size_t)sc->nx * sc->ny * sc->nz;
-  const size_t need = nvox * sizeof(float4) + 256u;  // the quads, then DiffGrid::zc
+  const size_t need = nvox * sizeof(float4);
   if (c->diff_quad_bytes < need) {  // grow; earlier work on the old buffer must finish first
     R3D_CUDA_TRY(c, cudaDeviceSynchronize());
     cudaFree(c->diff_quad);
@@ -746,10 +780,8 @@ static int diff_quads(r3d_cuda_ctx *c, const r3d_cuda_diff_scene *sc, DiffGrid &
     c->diff_quad_bytes = need;
   }
   g.quad = (const float4 *)c->diff_quad;
-  uint32_t *zc = (uint32_t *)((char *)c->diff_quad + nvox * sizeof(float4));
-  g.zc = zc;
   // the TF may change between calls that share the density
-  k_diff_tf_clear<<<1, 256, 0, st>>>(sc->lut, zc);
+  k_diff_tf_clear<<<1, 256, 0, st>>>(sc->lut, g.zc);
   R3D_CUDA_TRY(c, cudaGetLastError());
   if (reuse && c->quad_src == sc->density) return R3D_OK;
   k_diff_quads<<<grid_blocks(nvox), 256, 0, st>>>(sc->density, sc->nx, sc->ny, sc->nz,
@@ -780,7 +812,9 @@ static int diff_forward(r3d_cuda_ctx *c, const r3d_cuda_diff_scene *sc,
   DiffView *dv;
   uint32_t nt;
   size_t nf;
-  int rc = diff_prepare(c, sc, views, nviews, g, dv, nt, nf, st);
+  int slot = 0;
+  bool captured = false;
+  int rc = diff_prepare(c, sc, views, nviews, g, dv, nt, nf, slot, captured, st);
   if (rc != R3D_OK) return rc;
   rc = diff_quads(c, sc, g, false, st);
   if (rc != R3D_OK) return rc;
@@ -811,6 +845,8 @@ static int diff_forward(r3d_cuda_ctx *c, const r3d_cuda_diff_scene *sc,
     k_diff_fwd<false><<<march_blocks(k_diff_fwd<false>, nt), 128, 0, st>>>(
         dv, nviews, nt, g, rgb_out, total_steps, nullptr, nullptr);
   R3D_CUDA_TRY(c, cudaGetLastError());
+  rc = call_marched(c, slot, captured, st);
+  if (rc != R3D_OK) return rc;
   R3D_CUDA_TRY(c, cudaEventRecord(c->ev1, st));
   c->timed = true;
   if (tape) {
@@ -869,7 +905,9 @@ extern "C" int r3d_cuda_raycast_bwd(r3d_cuda_ctx *c, const r3d_cuda_diff_scene *
   DiffView *dv;
   uint32_t nt;
   size_t nf;
-  int rc = diff_prepare(c, sc, views, nviews, g, dv, nt, nf, st);
+  int slot = 0;
+  bool captured = false;
+  int rc = diff_prepare(c, sc, views, nviews, g, dv, nt, nf, slot, captured, st);
   if (rc != R3D_OK) return rc;
   const size_t nvox = (size_t)sc->nx * sc->ny * sc->nz;
   unsigned long long *qd = nullptr, *ql = nullptr, *qs = nullptr;
@@ -914,6 +952,8 @@ extern "C" int r3d_cuda_raycast_bwd(r3d_cuda_ctx *c, const r3d_cuda_diff_scene *
                         : launch_bwd<128, false>(nviews, nt, st, dv, g, dl_drgb, gd, qd, gl, ql, gs, qs, tp, tn);
   }
   if (e != cudaSuccess) return cuda_fail(c, e, "raycast_bwd: launch");
+  rc = call_marched(c, slot, captured, st);
+  if (rc != R3D_OK) return rc;
   if (det) {
     k_fix_to_float<<<grid_blocks(nvox), 256, 0, st>>>(qd, gd, nvox);
     k_fix_to_float<<<4, 256, 0, st>>>(ql, gl, 1024);

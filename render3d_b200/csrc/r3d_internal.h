@@ -181,6 +181,14 @@ struct r3d_cuda_ctx {
   cudaEvent_t ring_ev[kRing] = {};
   bool ring_used[kRing] = {};
   int ring_next = 0;
+  // two words per ring slot of the differentiable calls (call_words), and
+  // after them those of captured calls; ring_march_ev[k] completes once the
+  // march of the slot's last such call has run
+  static constexpr uint32_t kCapturedCalls = 1024u;
+  uint32_t *diff_words = nullptr;
+  uint32_t captured_next = 0;
+  cudaEvent_t ring_march_ev[kRing] = {};
+  bool ring_marched[kRing] = {};
 
   r3d::DevScene scene() const;
 };
