@@ -45,6 +45,18 @@ bool readable_in_place(const r3d_cuda_ctx *c, const void *p) {
   return a.type == cudaMemoryTypeDevice && a.device == c->device;
 }
 
+cudaError_t idle_device(r3d_cuda_ctx *c) {
+  if (!c->spare && cudaMalloc(&c->spare, 256u) != cudaSuccess) {
+    cudaGetLastError();
+    return cudaDeviceSynchronize();
+  }
+  const cudaError_t e = cudaFree(c->spare);
+  if (e != cudaSuccess) return e;
+  c->spare = nullptr;
+  if (cudaMalloc(&c->spare, 256u) != cudaSuccess) cudaGetLastError();  // taken next time
+  return cudaSuccess;
+}
+
 // ------------------------------------------------------------- builders
 
 // 26-neighbour max dilation (src/vk/vkbackend.c:845-860)
@@ -69,8 +81,8 @@ __global__ void k_occ_dilate(const uint8_t *__restrict__ raw, uint8_t *__restric
 
 
 template <class T>
-static cudaError_t reserve(T *&p, size_t &cap, size_t need) {
-  if (keeps(p, cap, need)) return cudaDeviceSynchronize();
+static cudaError_t reserve(r3d_cuda_ctx *c, T *&p, size_t &cap, size_t need) {
+  if (keeps(p, cap, need)) return idle_device(c);
   cudaFree(p);
   p = nullptr;
   cap = 0;
@@ -121,6 +133,7 @@ int r3d_cuda_create(int device, r3d_cuda_ctx **out) {
       cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaMalloc(&c->status, sizeof(uint32_t)) != cudaSuccess ||
       cudaMalloc(&c->lut, 256 * sizeof(uchar4)) != cudaSuccess ||
+      cudaMalloc(&c->spare, 256u) != cudaSuccess ||
       cudaMalloc(&c->total, (R3D_COUNTERS + 1) * sizeof(unsigned long long)) != cudaSuccess ||
       cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
       cudaMallocHost(&c->ring_host, sizeof(DevView) * kMaxBatchViews * r3d_cuda_ctx::kRing) !=
@@ -177,6 +190,7 @@ void r3d_cuda_destroy(r3d_cuda_ctx *c) {
   cudaFree(c->shard_buf);
   cudaFree(c->shard_page);
   cudaFree(c->lut);
+  cudaFree(c->spare);
   cudaFree(c->status);
   cudaFree(c->img);
   cudaFree(c->aux_buf);
@@ -254,7 +268,7 @@ int r3d_cuda_upload_volume(r3d_cuda_ctx *c, const r3d_volume_desc *d, const uint
   const size_t base = (total + onb + 255) & ~(size_t)255, qbytes = cube_quad_bytes(cube);
   const bool kept = keeps(c->cube_buf, c->cube_cap, base + qbytes);
   bool whole = true;
-  cudaError_t e = kept ? cudaDeviceSynchronize() : cudaMalloc(&buf, base + qbytes);
+  cudaError_t e = kept ? idle_device(c) : cudaMalloc(&buf, base + qbytes);
   if (e == cudaErrorMemoryAllocation && qbytes) {
     cudaGetLastError();
     whole = false;
@@ -391,8 +405,8 @@ static int reserve_tables(r3d_cuda_ctx *c) {
   c->br.bmax = nullptr;
   c->br.quad = nullptr;
   const size_t n = c->nslots ? c->nslots : 1u;
-  R3D_CUDA_TRY(c, reserve(c->bmax, c->bmax_cap, n * 4096u));
-  R3D_CUDA_TRY(c, reserve(c->quad, c->quad_cap, n * (128u * 128u * 128u) * sizeof(uint32_t)));
+  R3D_CUDA_TRY(c, reserve(c, c->bmax, c->bmax_cap, n * 4096u));
+  R3D_CUDA_TRY(c, reserve(c, c->quad, c->quad_cap, n * (128u * 128u * 128u) * sizeof(uint32_t)));
   if (!c->nslots) R3D_CUDA_TRY(c, cudaMemsetAsync(c->bmax, 0, 4096u, c->stream));
   return R3D_OK;
 }
@@ -411,7 +425,7 @@ int build_blockmax(r3d_cuda_ctx *c) {
 
 int replace_pool(r3d_cuda_ctx *c, uint32_t nslots) {
   c->br.pool = nullptr;
-  R3D_CUDA_TRY(c, reserve(c->pool, c->pool_cap, (size_t)(nslots ? nslots : 1u) * (128u * 128u * 128u)));
+  R3D_CUDA_TRY(c, reserve(c, c->pool, c->pool_cap, (size_t)(nslots ? nslots : 1u) * (128u * 128u * 128u)));
   c->br.pool = c->pool;
   return R3D_OK;
 }
@@ -539,7 +553,7 @@ int r3d_cuda_bricks_build(r3d_cuda_ctx *c, const r3d_volume_desc *d, const uint8
     // the pool and the page table: kept when about this size, else allocated
     // before the old ones go
     pool_bytes = (size_t)(nslots ? nslots : 1u) * (128u * 128u * 128u);
-    if (!keeps(c->pool, c->pool_cap, pool_bytes)) e = cudaMalloc(&pool, pool_bytes);
+    e = keeps(c->pool, c->pool_cap, pool_bytes) ? idle_device(c) : cudaMalloc(&pool, pool_bytes);
     if (e == cudaSuccess) e = cudaMalloc(&page, (size_t)words * 4);
     if (e != cudaSuccess) {
       rc = cuda_fail(c, e, "bricks_build: cudaMalloc pool");
@@ -551,8 +565,6 @@ int r3d_cuda_bricks_build(r3d_cuda_ctx *c, const r3d_volume_desc *d, const uint8
       c->pool = pool;
       c->pool_cap = pool_bytes;
       pool = nullptr;
-    } else {
-      e = cudaDeviceSynchronize();  // frames on other streams may read the old slots
     }
     cudaFree(c->page);
     c->page = page;

@@ -13,6 +13,7 @@
 struct r3d_cuda_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
+  void *spare = nullptr;  // idle_device
   std::string err;
 
   // cube volume: all mip levels in one allocation, then the occupancy grid
@@ -199,11 +200,16 @@ namespace r3d {
 // one of at least `need` and less than twice that many bytes is used again
 // (a 1024^3 brick cache's cudaMalloc and cudaFree calls took 10 ms of a rebuild's
 // 23), any other is replaced.  Frames in flight on other streams may still
-// read a kept buffer, so the device is idle before it is written again, as
-// cudaFree leaves it too.
+// read a kept buffer, so it is written again only after idle_device.
 inline bool keeps(const void *p, size_t cap, size_t need) {
   return p && cap >= need && need > cap / 2;
 }
+// Waits for the work of every stream of the device, as freeing a replaced
+// buffer does: by freeing the context's spare small one and taking it again
+// (4 us; an extra allocation for it could need a new 2 MB block of the
+// driver's each time, 0.6 ms).  cudaDeviceSynchronize would be refused while
+// another thread captures a stream, and end that capture; frees are not.
+cudaError_t idle_device(r3d_cuda_ctx *c);
 
 int fail(r3d_cuda_ctx *c, int code, const char *fmt, ...);
 int cuda_fail(r3d_cuda_ctx *c, cudaError_t e, const char *what);

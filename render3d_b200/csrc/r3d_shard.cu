@@ -136,7 +136,7 @@ int r3d_cuda_shard_build(r3d_cuda_ctx *c, uint32_t edge, const uint8_t *voxels, 
   const size_t base = (total + onb + 255) & ~(size_t)255, qbytes = cube_quad_bytes(h.atlas);
   const bool kept = keeps(c->shard_buf, c->shard_cap, base + qbytes);
   bool whole = true;
-  cudaError_t e = kept ? cudaDeviceSynchronize() : cudaMalloc(&buf, base + qbytes);
+  cudaError_t e = kept ? idle_device(c) : cudaMalloc(&buf, base + qbytes);
   if (e == cudaErrorMemoryAllocation && qbytes) {
     cudaGetLastError();
     whole = false;
