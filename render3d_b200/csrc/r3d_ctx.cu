@@ -275,12 +275,11 @@ int r3d_cuda_upload_volume(r3d_cuda_ctx *c, const r3d_volume_desc *d, const uint
     e = cudaMalloc(&buf, base);
   }
   if (e != cudaSuccess) return cuda_fail(c, e, "upload_volume: cudaMalloc");
-  if (kept) {
-    buf = c->cube_buf;
-    c->have_cube = false;
-  }
+  if (kept) buf = c->cube_buf;
   raw = buf + total;
+  // (a copy that is refused leaves a kept buffer, and its volume, as it was)
   e = cudaMemcpyAsync(buf, voxels, (size_t)nx * ny * nz, cudaMemcpyDefault, c->stream);
+  if (kept && e == cudaSuccess) c->have_cube = false;
   for (uint32_t m = 0; m < mips; m++) cube.lev[m] = buf + off[m];
   cube.occ = buf + off[mips];
   for (uint32_t m = 1; m < mips && e == cudaSuccess; m++)

@@ -279,6 +279,7 @@ void stream_reset(r3d_cuda_ctx *c);
 // linear pool of 128^3 slots (atlas_bpa 0) or of a single-level atlas of
 // atlas_bpa^3 slots.
 bool postfilter_on(const r3d_cuda_ctx *c, uint32_t target);
+cudaError_t postfilter_reserve(r3d_cuda_ctx *c);  // the scratch slots
 int postfilter_slots(r3d_cuda_ctx *c, uint32_t target, uint8_t *pool, const uint32_t *slots,
                      uint32_t n, uint32_t atlas_bpa = 0u);
 void postfilter_reset(r3d_cuda_ctx *c);

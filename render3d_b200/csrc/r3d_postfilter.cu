@@ -261,12 +261,16 @@ bool postfilter_on(const r3d_cuda_ctx *c, uint32_t target) {
   return primary_kernel(c->pf_mode & 0xFFu) != nullptr || (c->pf_mode & 0x100u);
 }
 
+cudaError_t postfilter_reserve(r3d_cuda_ctx *c) {
+  return c->pf_scratch ? cudaSuccess : cudaMalloc(&c->pf_scratch, (size_t)kPfWave * kSlotBytes);
+}
+
 int postfilter_slots(r3d_cuda_ctx *c, uint32_t target, uint8_t *pool, const uint32_t *slots,
                      uint32_t n, uint32_t atlas_bpa) {
   if (!n || !postfilter_on(c, target)) return R3D_OK;
   const PfKernel prim = primary_kernel(c->pf_mode & 0xFFu);
   const bool sharpen = (c->pf_mode & 0x100u) != 0;
-  if (!c->pf_scratch) R3D_CUDA_TRY(c, cudaMalloc(&c->pf_scratch, (size_t)kPfWave * kSlotBytes));
+  R3D_CUDA_TRY(c, postfilter_reserve(c));
   cudaStream_t st = c->stream;
   const dim3 grid(4u * 16u * 16u, 1u);
   for (uint32_t w0 = 0; w0 < n; w0 += kPfWave) {

@@ -155,6 +155,9 @@ int r3d_cuda_shard_build(r3d_cuda_ctx *c, uint32_t edge, const uint8_t *voxels, 
     e = cudaMemcpyAsync(dbrick, brick.data(), sizeof(uint32_t) * ns, cudaMemcpyHostToDevice,
                         c->stream);
   std::vector<uint32_t> maxv(nb);
+  // whatever else can be refused comes before a kept buffer, and its shard,
+  // is given up
+  if (e == cudaSuccess && postfilter_on(c, 0u)) e = postfilter_reserve(c);
   if (e == cudaSuccess) {
     if (kept) {
       buf = c->shard_buf;
