@@ -42,7 +42,8 @@ __global__ void __launch_bounds__(256) k_level_down(const uint8_t *__restrict__ 
       for (uint32_t k = 0; k < 4u; k++) {
         const uint32_t y = 2u * oy + (k & 1u), z = 2u * oz + (k >> 1);
         uint2 w = make_uint2(0u, 0u);
-        if (y < sy && z < sz) w = load8<VEC>(src + ((size_t)z * sy + y) * sx, 2u * ox, sx);
+        if (y < sy && z < sz)
+          w = load8<VEC>(src + ((size_t)z * sy + y) * sx, 2u * ox, sx, VEC || inner_row(y, z, sx, sy, sz));
         s0 += (w.x & 0x00FF00FFu) + ((w.x >> 8) & 0x00FF00FFu);
         s1 += (w.y & 0x00FF00FFu) + ((w.y >> 8) & 0x00FF00FFu);
         m = __vmaxu4(m, __vmaxu4(w.x, w.y));
@@ -137,7 +138,7 @@ __global__ void __launch_bounds__(256) k_slot_fill(const __grid_constant__ FillJ
       r[i] = 0u;
       if (z0 + z < ez && y0 + y < ey) {
         const uint8_t *row = g + ((size_t)(z0 + z) * ey + (y0 + y)) * ex;
-        r[i] = load4<VEC>(row, x0 + lane * 4u, ex);
+        r[i] = load4<VEC>(row, x0 + lane * 4u, ex, VEC || inner_row(y0 + y, z0 + z, ex, ey, ez));
       }
     }
 #pragma unroll

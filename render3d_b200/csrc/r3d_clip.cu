@@ -137,8 +137,8 @@ int r3d_cuda_clip_build(r3d_cuda_ctx *c, const r3d_volume_desc *d, const uint8_t
   const size_t vbytes = (size_t)nx * ny * nz;
   const size_t l1 = (size_t)c->clip_pyr_dim[1][0] * c->clip_pyr_dim[1][1] * c->clip_pyr_dim[1][2];
   uint8_t *half = nullptr;
-  cudaError_t e = cudaMalloc(&c->clip_src, vbytes);
-  if (e == cudaSuccess) e = cudaMalloc(&c->clip_pyr, pyr ? pyr : 1u);
+  cudaError_t e = cudaMalloc(&c->clip_src, vbytes + 4u);  // + 4: load4
+  if (e == cudaSuccess) e = cudaMalloc(&c->clip_pyr, pyr + 4u);
   if (e == cudaSuccess) e = cudaMalloc(&c->clip_tex, tex);
   if (e == cudaSuccess) e = cudaMalloc(&half, l1 ? l1 : 1u);
   if (e == cudaSuccess) e = copy_sync(c->stream, c->clip_src, voxels, vbytes);

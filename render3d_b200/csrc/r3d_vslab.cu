@@ -233,7 +233,7 @@ int r3d_cuda_vslab_begin(r3d_cuda_ctx *c, const r3d_volume_desc *d, const uint8_
   }
   c->vs_strip_bytes = strip;
   const uint32_t nslot = v.gx[0] * v.gy[0];
-  cudaError_t e = cudaMalloc(&c->vs_src, vbytes);
+  cudaError_t e = cudaMalloc(&c->vs_src, vbytes + 4u);  // + 4: load4
   if (e == cudaSuccess) e = cudaMalloc(&c->vs_tiles, tbytes * v.ntiles);
   c->vs_batch = v.gx[1] ? kVsBatch : 1u;  // strips of a whole batch, else of one job
   if (e == cudaSuccess && cudaMalloc(&c->vs_strip, strip * c->vs_batch) != cudaSuccess) {
