@@ -927,7 +927,7 @@ static int launch_views_persistent(r3d_cuda_ctx *c, uint32_t persistent,
     L.path = (int)(gkey[g] >> 3);
     int per_sm = sc.blocks_per_sm
                      ? (int)sc.blocks_per_sm
-                     : persist_blocks_per_sm(L.path, L.mode, L.fast, L.unroll);
+                     : persist_blocks_per_sm(L, s);
     // no more blocks than there are tiles for their warps
     uint32_t want = (uint32_t)per_sm * (uint32_t)dev_sms;
     uint32_t cap = (L.ntiles + 3u) / 4u;

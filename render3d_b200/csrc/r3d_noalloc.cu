@@ -177,7 +177,7 @@ extern "C" int r3d_cuda_raycast_fwd_noalloc(r3d_cuda_ctx *c, const r3d_frame_par
     L.path = (int)(gkey[g] >> 3);
     const int per_sm = sc.blocks_per_sm
                            ? (int)sc.blocks_per_sm
-                           : persist_blocks_per_sm(L.path, L.mode, L.fast, L.unroll);
+                           : persist_blocks_per_sm(L, s);
     uint32_t want = (uint32_t)per_sm * (uint32_t)sms;
     uint32_t cap = (L.ntiles + 3u) / 4u;
     L.blocks = want < cap ? want : (cap ? cap : 1u);

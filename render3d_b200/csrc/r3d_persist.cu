@@ -372,37 +372,29 @@ static cudaError_t launch_tm(const TilesLaunch &L, cudaStream_t st) {
   }
 }
 
-template <int PATH, int MODE, bool FAST, bool COUNT, int UNROLL>
-static cudaError_t launch_pt(const PersistLaunch &L, const DevScene &s, cudaStream_t st) {
-  k_raycast_persist<PATH, MODE, FAST, COUNT, UNROLL><<<L.blocks, 128, 0, st>>>(
-      L.views, L.nviews, s, L.lut, L.queue, L.ntiles, L.refill_min, L.shape, L.steps, L.mip,
-      L.total, L.counters);
-  return cudaGetLastError();
-}
-
-template <int PATH, int MODE, bool FAST, bool COUNT>
-static cudaError_t launch_pu(const PersistLaunch &L, const DevScene &s, cudaStream_t st) {
-  return L.unroll == 2 ? launch_pt<PATH, MODE, FAST, COUNT, 2>(L, s, st)
-                       : launch_pt<PATH, MODE, FAST, COUNT, 1>(L, s, st);
-}
+// The lane-refill kernel of a mode (all of one signature).
+using PersistKernel = decltype(&k_raycast_persist<PATH_CUBE, R3D_MODE_MIP, false, false, 1>);
 
 template <int PATH, int MODE, bool FAST>
-static cudaError_t launch_pc(const PersistLaunch &L, const DevScene &s, cudaStream_t st) {
-  return L.counters ? launch_pu<PATH, MODE, FAST, true>(L, s, st)
-                    : launch_pu<PATH, MODE, FAST, false>(L, s, st);
+static PersistKernel persist_kernel_of(bool count, uint32_t unroll) {
+  if (count)
+    return unroll == 2u ? &k_raycast_persist<PATH, MODE, FAST, true, 2>
+                        : &k_raycast_persist<PATH, MODE, FAST, true, 1>;
+  return unroll == 2u ? &k_raycast_persist<PATH, MODE, FAST, false, 2>
+                      : &k_raycast_persist<PATH, MODE, FAST, false, 1>;
 }
 
 template <int PATH>
-static cudaError_t launch_pm(const PersistLaunch &L, const DevScene &s, cudaStream_t st) {
-  switch (L.mode) {
+static PersistKernel persist_kernel(uint32_t mode, bool fast, bool count, uint32_t unroll) {
+  switch (mode) {
     case R3D_MODE_FULL:
-      return L.fast ? launch_pc<PATH, R3D_MODE_FULL, true>(L, s, st)
-                    : launch_pc<PATH, R3D_MODE_FULL, false>(L, s, st);
-    case R3D_MODE_MIP: return launch_pc<PATH, R3D_MODE_MIP, false>(L, s, st);
-    case R3D_MODE_DEPTH: return launch_pc<PATH, R3D_MODE_DEPTH, false>(L, s, st);
-    case R3D_MODE_HEATMAP: return launch_pc<PATH, R3D_MODE_HEATMAP, false>(L, s, st);
-    case R3D_MODE_RAYDIR: return launch_pc<PATH, R3D_MODE_RAYDIR, false>(L, s, st);
-    default: return launch_pc<PATH, R3D_MODE_FLAT, false>(L, s, st);
+      return fast ? persist_kernel_of<PATH, R3D_MODE_FULL, true>(count, unroll)
+                  : persist_kernel_of<PATH, R3D_MODE_FULL, false>(count, unroll);
+    case R3D_MODE_MIP: return persist_kernel_of<PATH, R3D_MODE_MIP, false>(count, unroll);
+    case R3D_MODE_DEPTH: return persist_kernel_of<PATH, R3D_MODE_DEPTH, false>(count, unroll);
+    case R3D_MODE_HEATMAP: return persist_kernel_of<PATH, R3D_MODE_HEATMAP, false>(count, unroll);
+    case R3D_MODE_RAYDIR: return persist_kernel_of<PATH, R3D_MODE_RAYDIR, false>(count, unroll);
+    default: return persist_kernel_of<PATH, R3D_MODE_FLAT, false>(count, unroll);
   }
 }
 
@@ -412,7 +404,10 @@ static cudaError_t launch_pm(const PersistLaunch &L, const DevScene &s, cudaStre
 template <>
 cudaError_t persist_path<R3D_FWD_PATH>(const PersistLaunch &L, const DevScene &s,
                                        cudaStream_t st) {
-  return launch_pm<R3D_FWD_PATH>(L, s, st);
+  persist_kernel<R3D_FWD_PATH>(L.mode, L.fast, L.counters != nullptr, L.unroll)
+      <<<L.blocks, 128, 0, st>>>(L.views, L.nviews, s, L.lut, L.queue, L.ntiles, L.refill_min, L.shape,
+                                 L.steps, L.mip, L.total, L.counters);
+  return cudaGetLastError();
 }
 
 template <>
@@ -420,22 +415,16 @@ cudaError_t tiles_path<R3D_FWD_PATH>(const TilesLaunch &L, cudaStream_t st) {
   return launch_tm<R3D_FWD_PATH>(L, st);
 }
 
+// Resident blocks of the very kernel that a launch takes: with the FULL
+// kernel's (96 registers, 5 blocks) for every mode, the virtual slab's MIP and
+// step views (64 registers, 8 blocks) drained 400 x 300 pixels in 85 us, 64 now;
+// the quad paths' with the byte kernels', a 512^3 atlas 2.41 ms MIP, 2.05 now.
 template <>
-int persist_occupancy<R3D_FWD_PATH>(uint32_t mode, bool fast, uint32_t unroll) {
-  // occupancy of the instantiation that persist_path picks
-  constexpr int P = R3D_FWD_PATH;
+int persist_occupancy<R3D_FWD_PATH>(const PersistLaunch &L) {
   int n = 0;
-  cudaError_t e;
-  if (P == PATH_LOD_BRICKS && (mode != R3D_MODE_FULL || fast))
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &n, k_raycast_persist<P, R3D_MODE_MIP, false, false, 1>, 128, 0);
-  else if (P == PATH_LOD_BRICKS && unroll == 2)
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &n, k_raycast_persist<P, R3D_MODE_FULL, false, false, 2>, 128, 0);
-  else
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &n, k_raycast_persist<P, R3D_MODE_FULL, false, false, 1>, 128, 0);
-  if (e != cudaSuccess) {
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+          &n, persist_kernel<R3D_FWD_PATH>(L.mode, L.fast, L.counters != nullptr, L.unroll), 128, 0) !=
+      cudaSuccess) {
     cudaGetLastError();
     return 4;
   }
@@ -468,14 +457,16 @@ cudaError_t launch_tiles(const TilesLaunch &L, cudaStream_t st) {
   }
 }
 
-int persist_blocks_per_sm(int path, uint32_t mode, bool fast, uint32_t unroll) {
-  switch (path) {
-    case PATH_VSLAB: return persist_occupancy<PATH_VSLAB>(mode, fast, unroll);
-    case PATH_CLIP: return persist_occupancy<PATH_CLIP>(mode, fast, unroll);
-    case PATH_SLAB: return persist_occupancy<PATH_SLAB>(mode, fast, unroll);
-    case PATH_LOD_BRICKS: return persist_occupancy<PATH_LOD_BRICKS>(mode, fast, unroll);
-    case PATH_SHARD: return persist_occupancy<PATH_SHARD>(mode, fast, unroll);
-    default: return persist_occupancy<PATH_CUBE>(mode, fast, unroll);
+int persist_blocks_per_sm(const PersistLaunch &L, const DevScene &s) {
+  switch (quad_path(L.path, &s, 1u)) {
+    case PATH_VSLAB: return persist_occupancy<PATH_VSLAB>(L);
+    case PATH_CLIP: return persist_occupancy<PATH_CLIP>(L);
+    case PATH_SLAB: return persist_occupancy<PATH_SLAB>(L);
+    case PATH_LOD_BRICKS: return persist_occupancy<PATH_LOD_BRICKS>(L);
+    case PATH_SHARD: return persist_occupancy<PATH_SHARD>(L);
+    case PATH_SHARD_QUAD: return persist_occupancy<PATH_SHARD_QUAD>(L);
+    case PATH_CUBE_QUAD: return persist_occupancy<PATH_CUBE_QUAD>(L);
+    default: return persist_occupancy<PATH_CUBE>(L);
   }
 }
 #endif

@@ -78,11 +78,12 @@ cudaError_t launch_persist(const PersistLaunch &L, const DevScene &s, cudaStream
 cudaError_t launch_tiles(const TilesLaunch &L, cudaStream_t st);
 template <int PATH>
 cudaError_t tiles_path(const TilesLaunch &L, cudaStream_t st);
-int persist_blocks_per_sm(int path, uint32_t mode, bool fast, uint32_t unroll);
+// Resident blocks per SM of the kernel that launch_persist would take
+int persist_blocks_per_sm(const PersistLaunch &L, const DevScene &s);
 // Per-path halves of the two above (each defined in its own object).
 template <int PATH>
 cudaError_t persist_path(const PersistLaunch &L, const DevScene &s, cudaStream_t st);
 template <int PATH>
-int persist_occupancy(uint32_t mode, bool fast, uint32_t unroll);
+int persist_occupancy(const PersistLaunch &L);
 
 }  // namespace r3d

@@ -1,6 +1,7 @@
 """Runs a script in a child process with a few CUDA runtime calls behind a
-shim that can be told to refuse them: the failing calls of the tests that
-import this are error codes made on the host."""
+shim that can be told to refuse them, so that the failing calls of the tests
+that import this are error codes made on the host, and that notes the kernels
+launched and asked about."""
 import os
 import subprocess
 import sys
@@ -29,6 +30,30 @@ int cudaMemcpyAsync(void *d, const void *s, size_t n, int k, void *st) {
   if (copy_in > 0 && --copy_in == 0) { refused++; return 1; }  /* cudaErrorInvalidValue */
   return real(d, s, n, k, st);
 }
+typedef struct { unsigned x, y, z; } dim3_;
+static const void *launched[64];
+static unsigned grid[64], launches;
+static const void *asked;
+static int answer;
+unsigned shim_launches(void) { return launches; }
+const void *shim_kernel(unsigned k) { return launched[k % 64]; }
+unsigned shim_grid(unsigned k) { return grid[k % 64]; }
+const void *shim_asked(int *blocks) { *blocks = answer; return asked; }
+int cudaLaunchKernel(const void *f, dim3_ g, dim3_ b, void **a, size_t sm, void *st) {
+  static int (*real)(const void *, dim3_, dim3_, void **, size_t, void *);
+  if (!real) *(void **)&real = real_of("cudaLaunchKernel");
+  launched[launches % 64] = f;
+  grid[launches++ % 64] = g.x;
+  return real(f, g, b, a, sm, st);
+}
+int cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int *n, const void *f, int b, size_t sm,
+                                                           unsigned fl) {
+  static int (*real)(int *, const void *, int, size_t, unsigned);
+  if (!real) *(void **)&real = real_of("cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags");
+  const int e = real(n, f, b, sm, fl);
+  asked = f, answer = *n;
+  return e;
+}
 int cudaMalloc(void **p, size_t n) {
   static int (*real)(void **, size_t);
   if (!real) *(void **)&real = real_of("cudaMalloc");
@@ -44,6 +69,7 @@ import numpy as np
 import render3d_b200 as rb
 shim = ctypes.CDLL({so!r})
 shim.shim_alloc.argtypes = [ctypes.c_size_t, ctypes.c_size_t]
+shim.shim_kernel.restype = shim.shim_asked.restype = ctypes.c_void_p
 lut = rb.scroll_ramp_tf()
 W, H = 48, 40
 
