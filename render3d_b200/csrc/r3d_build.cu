@@ -356,6 +356,16 @@ size_t cube_quad_bytes(DevCube &c) {
   return words * sizeof(uint32_t);
 }
 
+bool words_fit(size_t bytes, size_t words, size_t back) {
+  size_t left = 0, all = 0;
+  if (words <= (size_t)1 << 30) return true;
+  if (cudaMemGetInfo(&left, &all) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return left + back >= bytes + words + all / 4u;
+}
+
 cudaError_t build_cube_quads(DevCube &c, uint32_t *at, cudaStream_t st) {
   c.quad = at;
   cudaError_t e = cudaSuccess;

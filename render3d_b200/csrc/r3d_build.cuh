@@ -116,6 +116,14 @@ cudaError_t launch_level_quads(const uint8_t *src, uint32_t dx, uint32_t dy, uin
 // kQuadVoxels), setting c.qoff; and the words themselves, at `at` (null:
 // none, the bytes are sampled), setting c.quad.
 size_t cube_quad_bytes(DevCube &c);
+// Whether `words` bytes of quad words may be taken with `bytes` bytes of
+// levels, `back` bytes being given back for them.  The words make a volume five
+// times as large, and what a program allocates after it should fit as it does
+// beside the bytes alone: so words of more than a gibibyte are taken only where
+// a quarter of the device's memory stays free (asking takes 0.09 ms, a fifth of
+// a small volume's first upload; without the words a view takes up to twice
+// as long).
+bool words_fit(size_t bytes, size_t words, size_t back);
 cudaError_t build_cube_quads(DevCube &c, uint32_t *at, cudaStream_t st);
 
 // Quad words and block maxima of slots slot[0..njobs) (null: 0..njobs) of a

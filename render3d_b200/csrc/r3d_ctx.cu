@@ -265,7 +265,10 @@ int r3d_cuda_upload_volume(r3d_cuda_ctx *c, const r3d_volume_desc *d, const uint
   // bytes, occupancy (and its raw grid) and quad words in one allocation,
   // kept when about this size as the brick cache's are; the words stand alone
   // when the whole does not fit beside the volume it replaces
-  const size_t base = (total + onb + 255) & ~(size_t)255, qbytes = cube_quad_bytes(cube);
+  const size_t base = (total + onb + 255) & ~(size_t)255;
+  size_t qbytes = cube_quad_bytes(cube);
+  if (!keeps(c->cube_buf, c->cube_cap, base + qbytes) && !words_fit(base, qbytes, c->cube_cap))
+    qbytes = 0;
   const bool kept = keeps(c->cube_buf, c->cube_cap, base + qbytes);
   bool whole = true;
   cudaError_t e = kept ? idle_device(c) : cudaMalloc(&buf, base + qbytes);

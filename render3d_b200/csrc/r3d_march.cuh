@@ -78,7 +78,7 @@ struct DevCube {
   // per texel of level m, from word qoff[m]: the bytes at (x, y), (x1, y),
   // (x, y1), (x1, y1) of its z plane, x1 = min(x + 1, dim - 1) and y1
   // likewise; nullptr when the volume is too large for them (kQuadVoxels) or
-  // they did not fit the memory
+  // they did not fit the memory (words_fit)
   const uint32_t *quad;
   uint32_t qoff[kMaxLevels];
 };

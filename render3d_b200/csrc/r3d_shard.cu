@@ -133,7 +133,10 @@ int r3d_cuda_shard_build(r3d_cuda_ctx *c, uint32_t edge, const uint8_t *voxels, 
   uint8_t *buf = nullptr, *vtmp = nullptr;
   uint32_t *dpage = nullptr;
   const bool dev_in = readable_in_place(c, voxels) && ((uintptr_t)voxels & 15u) == 0u;
-  const size_t base = (total + onb + 255) & ~(size_t)255, qbytes = cube_quad_bytes(h.atlas);
+  const size_t base = (total + onb + 255) & ~(size_t)255;
+  size_t qbytes = cube_quad_bytes(h.atlas);
+  if (!keeps(c->shard_buf, c->shard_cap, base + qbytes) && !words_fit(base, qbytes, c->shard_cap))
+    qbytes = 0;
   const bool kept = keeps(c->shard_buf, c->shard_cap, base + qbytes);
   bool whole = true;
   cudaError_t e = kept ? idle_device(c) : cudaMalloc(&buf, base + qbytes);

@@ -54,11 +54,24 @@ int cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int *n, const void *f
   asked = f, answer = *n;
   return e;
 }
+static size_t largest;
+size_t shim_largest(void) { size_t n = largest; largest = 0; return n; }
 int cudaMalloc(void **p, size_t n) {
   static int (*real)(void **, size_t);
   if (!real) *(void **)&real = real_of("cudaMalloc");
   if (n >= lo && n <= hi) { refused++; return 2; }  /* cudaErrorMemoryAllocation */
+  if (n > largest) largest = n;
   return real(p, n);
+}
+/* the device's free memory, as the library under test is told */
+static size_t left_free;
+void shim_free(size_t n) { left_free = n; }
+int cudaMemGetInfo(size_t *f, size_t *t) {
+  static int (*real)(size_t *, size_t *);
+  if (!real) *(void **)&real = real_of("cudaMemGetInfo");
+  const int e = real(f, t);
+  if (left_free) *f = left_free;
+  return e;
 }
 """
 
@@ -69,6 +82,8 @@ import numpy as np
 import render3d_b200 as rb
 shim = ctypes.CDLL({so!r})
 shim.shim_alloc.argtypes = [ctypes.c_size_t, ctypes.c_size_t]
+shim.shim_free.argtypes = [ctypes.c_size_t]
+shim.shim_largest.restype = ctypes.c_size_t
 shim.shim_kernel.restype = shim.shim_asked.restype = ctypes.c_void_p
 lut = rb.scroll_ramp_tf()
 W, H = 48, 40
