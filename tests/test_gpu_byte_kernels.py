@@ -87,3 +87,37 @@ vol = rb.phantom(256, seed=77)
 check(lambda x: x.shard_build(vol, 2, slots), vol.size, orc.ShardScene.build(vol, 2, slots),
       lambda x: x.shard_mode)
 """)
+
+
+@pytest.mark.parametrize("kind", ["cube", "shard"])
+def test_words_alone(tmp_path, kind):
+    """Where words do not fit in one allocation with the bytes they are
+    allocated alone, and go when the volume is replaced."""
+    run(tmp_path, BODY + f"""
+kind = {kind!r}
+vols = [rb.phantom(128, seed=k) for k in (1, 2, 3)]
+
+def build(x, k):
+    x.upload_volume(vols[k]) if kind == "cube" else x.shard_build(vols[k])
+    return x.shard_mode if kind == "shard" else 0
+
+d = rb.Context(0)
+d.set_transfer(lut)
+want = []
+shim.shim_largest()
+for k in range(3):
+    p = view(rb.MODE_FULL, build(c, k))
+    want.append(draw(c, p, 0, 0)[:2])
+    if k == 0:
+        size = shim.shim_largest()
+for k, whole in enumerate((False, False, True)):
+    if not whole:
+        shim.shim_alloc(size, size)
+    build(d, k)
+    assert bool(shim.shim_refused()) != whole
+    shim.shim_alloc(1, 0)
+    got = draw(d, p, 0, 0)[:2]
+    assert got[0] == want[k][0], "another kernel"
+    assert np.array_equal(got[1], want[k][1])
+d.close()
+""")
