@@ -18,7 +18,7 @@ def test_words_lie_inside_the_row(tmp_path):
     src = tmp_path / "rows.c"
     src.write_text(SRC)
     so = str(tmp_path / "rows.so")
-    subprocess.run(["/usr/bin/gcc", "-O1", "-shared", "-fPIC", "-I" + os.path.join(ROOT, "include"), "-o", so,
+    subprocess.run(["/usr/bin/gcc", "-O1", "-shared", "-fPIC", "-I" + os.path.join(ROOT, "render3d_b200", "csrc"), "-o", so,
                     str(src)], check=True)
     lib = ctypes.CDLL(so)
     for start in range(4):  # the row's address
