@@ -537,7 +537,7 @@ int r3d_cuda_batch_launch(r3d_cuda_batch *batch, unsigned long long *total_steps
 int r3d_cuda_batch_capture(r3d_cuda_batch *batch, unsigned long long *total_steps, void *stream);
 int r3d_cuda_batch_replay(r3d_cuda_batch *batch, void *stream);
 /* Autotuner: times every candidate schedule (one thread per ray with
- * grouped shading off / 4 / 8 / 16; lane refill with tile 8x4 / 16x2 /
+ * shading batches of 32 / 4 / 8 / 16 samples; lane refill with tile 8x4 / 16x2 /
  * 32x1, refill threshold 8 / 16 / 24, 1 or 2 steps between refills, for a
  * batch of one scene; whole 8x4 tiles) over `reps` launches each after a
  * warm-up, keeps the fastest as the batch's schedule and returns it with
@@ -577,8 +577,9 @@ int r3d_cuda_diff_forward(r3d_cuda_ctx *ctx, const r3d_cuda_diff_scene *scene,
                           unsigned long long *total_steps, void *stream);
 
 /* The same render, recording a tape for the backward: per ray, the first 64
- * contributing samples (march position and the opacity accumulated before
- * them) and their count, in a context-owned buffer of 516 bytes per ray.
+ * contributing samples (march position, the opacity accumulated before it,
+ * the sample's density and opacity) and their count, in a context-owned buffer
+ * of 1028 bytes per ray, each view's extents rounded up to tiles of 8x4 rays.
  * A later r3d_cuda_raycast_bwd with R3D_BWD_TAPE over the same views and
  * scene (same buffers, sizes and cutoff) reads it instead of marching the
  * rays forward again; the grid and LUT contents must not change in
